@@ -72,6 +72,7 @@ struct IgemmArgs {
   const float* scale2;
   const float* bias2;
   int out_mode, ldy;
+  int nchw_words;                      // NCHW output: groups of four pixels are whole aligned words of an int8 plane
   void* y;
   const float* scale;
   const float* bias;
@@ -310,6 +311,81 @@ __device__ __forceinline__ void epilogue_chunk_staged(const IgemmArgs& a, const 
   }
   sts128(st_b_row + (((byte_chunk0) ^ b_swz_mask) << 4), q[0], q[1], q[2], q[3]);
   sts128(st_b_row + (((byte_chunk0 + 1) ^ b_swz_mask) << 4), q[4], q[5], q[6], q[7]);
+}
+
+// ---------------------------------------------------------------- epilogue into NCHW tensors
+// A lane owns one pixel, so the 32 lanes of a warp hold 32 consecutive pixels of every channel: written channel by
+// channel the accumulator tile IS the NCHW layout.  fp32 / int32 values leave as one full 128-byte row segment per
+// channel; int8 values are transposed four pixels x four channels at a time inside groups of four lanes (two shuffles
+// per four words) and leave as words, or, where a plane's rows are not whole words, byte by byte.  This replaces a
+// channels-last output tensor in the workspace and a transposing pass over it.
+// Four words of four channels (word j = channels 4j .. 4j+3 of this lane's pixel) -> four words of four pixels
+// (word j = this group's pixels 0..3 of channel 4j + (lane & 3)).
+__device__ __forceinline__ void transpose_bytes_across4(uint32_t (&q)[8], int lane) {
+  const bool b1 = (lane & 2) != 0, b0 = (lane & 1) != 0;
+  const uint32_t s_send1 = b1 ? 0x5410u : 0x7632u;
+  const uint32_t s_send0 = b0 ? 0x6420u : 0x7531u, s_a0 = b0 ? 0x3514u : 0x5240u, s_b0 = b0 ? 0x3716u : 0x7260u;
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) {
+    // partner two pixels away: lanes 0, 1 keep channels 0, 1 of both pixels, lanes 2, 3 channels 2, 3
+    uint32_t recv = __shfl_xor_sync(0xffffffffu, __byte_perm(q[j], q[j + 1], s_send1), 2);
+    // (low half = the lower pixel; for lanes 2, 3 that is the received one)
+    const uint32_t ta = b1 ? __byte_perm(recv, q[j], 0x7610u) : __byte_perm(q[j], recv, 0x5410u);
+    const uint32_t tb = b1 ? __byte_perm(recv, q[j + 1], 0x7632u) : __byte_perm(q[j + 1], recv, 0x7610u);
+    recv = __shfl_xor_sync(0xffffffffu, __byte_perm(ta, tb, s_send0), 1);
+    q[j] = __byte_perm(ta, recv, s_a0);
+    q[j + 1] = __byte_perm(tb, recv, s_b0);
+  }
+}
+
+// One 32-column chunk.  `off` = element offset of (this lane's pixel, channel `col`); planes are `hw` elements apart.
+template <int MODE, int ACT>
+__device__ __forceinline__ void epilogue_nchw32(const IgemmArgs& a, const float* scale, const float* bias, const uint32_t (&r)[32],
+                                                int lane, int col, bool valid, long off, long hw) {
+  const int ncols = a.cout - col < 32 ? a.cout - col : 32;
+  const float4* sc4 = reinterpret_cast<const float4*>(scale + col);
+  const float4* bi4 = reinterpret_cast<const float4*>(bias + col);
+  if (MODE == OUT_I8) {
+    const float ub = quant_upper_bound<ACT>(a.alpha);
+    uint32_t q[8];
+    if (a.acc_small) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) q[j] = quant4<ACT, true>(&r[4 * j], sc4[j], bi4[j], a.alpha, ub);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) q[j] = quant4<ACT, false>(&r[4 * j], sc4[j], bi4[j], a.alpha, ub);
+    }
+    int8_t* dst = static_cast<int8_t*>(a.y) + off;
+    if (a.nchw_words) {
+      transpose_bytes_across4(q, lane);
+      const int i = lane & 3;
+      dst += i * hw - i;  // channel i of the group, first pixel of the group
+      const long step = 4 * hw;
+#pragma unroll
+      for (int j = 0; j < 8; ++j, dst += step)
+        if (valid && 4 * j + i < ncols) *reinterpret_cast<uint32_t*>(dst) = q[j];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j, dst += hw)
+        if (valid && j < ncols) *dst = static_cast<int8_t>(q[j >> 2] >> (8 * (j & 3)));
+    }
+    return;
+  }
+  uint32_t* dst = static_cast<uint32_t*>(a.y) + off;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    uint32_t v[4] = {r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]};
+    if (MODE == OUT_F32) {
+      const float4 sc = sc4[j], bi = bi4[j];
+      v[0] = __float_as_uint(act_f32<ACT>(fmaf(__int2float_rn((int)v[0]), sc.x, bi.x), a.alpha));
+      v[1] = __float_as_uint(act_f32<ACT>(fmaf(__int2float_rn((int)v[1]), sc.y, bi.y), a.alpha));
+      v[2] = __float_as_uint(act_f32<ACT>(fmaf(__int2float_rn((int)v[2]), sc.z, bi.z), a.alpha));
+      v[3] = __float_as_uint(act_f32<ACT>(fmaf(__int2float_rn((int)v[3]), sc.w, bi.w), a.alpha));
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e, dst += hw)
+      if (valid && 4 * j + e < ncols) *dst = v[e];
+  }
 }
 
 // ---------------------------------------------------------------- MMA issue sequences
@@ -577,7 +653,9 @@ __device__ __forceinline__ bool mma_loop_window_resident(const IgemmArgs& a, uin
 // side by side hit the same activation rows in L2.  The operand ring and the TMEM
 // accumulator buffers run across tile boundaries: the producer prefetches the next tiles
 // while the epilogue groups drain the previous ones.
-template <int MODE, int ACT, bool STAGED>
+enum Store : int { STORE_DIRECT = 0, STORE_STAGED = 1, STORE_NCHW = 2 };
+
+template <int MODE, int ACT, int STORE>
 __global__ void __launch_bounds__(kThreads, 1)
     igemm_i8_tc_kernel(const __grid_constant__ CUtensorMap tmA,
                        const __grid_constant__ CUtensorMap tmB,
@@ -586,6 +664,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                        const __grid_constant__ CUtensorMap tmOutB,
                        const __grid_constant__ CUtensorMap tmA2,
                        const __grid_constant__ CUtensorMap tmB2, const IgemmArgs a) {
+  constexpr bool STAGED = STORE == STORE_STAGED;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem_al = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -1191,6 +1270,38 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           stores_pending = true;
         }
+      } else if (STORE == STORE_NCHW) {
+        // this lane's pixel of the [batch, cout, ho, wo] output
+        const int hw = a.ho * a.wo;
+        int img, pix;
+        bool valid;
+        if (a.slab) {
+          const int tile_m = tile / a.tiles_n;
+          const int t = tile_m / a.tiles_x;
+          const int px = (tile_m % a.tiles_x) * 8 + (lane & 7), py = (t % a.tiles_y) * 16 + quad * 4 + (lane >> 3);
+          img = t / a.tiles_y;
+          pix = py * a.wo + px;
+          valid = px < a.wo && py < a.ho;
+        } else {
+          const int m = m0 + quad * 32 + lane;
+          img = m / hw;
+          pix = m - img * hw;
+          valid = m < a.m_total;
+        }
+        const long base = static_cast<long>(img) * a.cout * hw + pix;
+        for (int c = col_par * 32; c < a.bn; c += 32 * gpb) {
+          if (n0 + c >= a.cout) break;  // warp-uniform
+          if (!waited) {
+            ok = mbar_wait(smem_u32(&acc_full[my_buf]), (it >> nb_shift) & 1, abort_flag, a.status, FAULT_WAIT_ACCUM);
+            tc_fence_after();
+            waited = true;
+            if (!ok) break;
+          }
+          uint32_t r[32];
+          tc_ld32(lane_addr + static_cast<uint32_t>(c), r);
+          tc_wait_ld();
+          epilogue_nchw32<MODE, ACT>(a, ep_scale, ep_bias, r, lane, n0 + c, valid, base + static_cast<long>(n0 + c) * hw, hw);
+        }
       } else {
         for (int c = col_par * 32; c < a.bn; c += 32 * gpb) {
           if (n0 + c >= a.cout) break;  // warp-uniform
@@ -1245,28 +1356,33 @@ __global__ void __launch_bounds__(kThreads, 1)
 typedef void (*IgemmKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                             const CUtensorMap, const CUtensorMap, const CUtensorMap, const IgemmArgs);
 
-template <int MODE, bool STAGED>
+template <int MODE, int STORE>
 IgemmKernel pick_act(int act) {
   switch (act) {
-    case PLB_ACT_RELU: return igemm_i8_tc_kernel<MODE, PLB_ACT_RELU, STAGED>;
-    case PLB_ACT_RELU6: return igemm_i8_tc_kernel<MODE, PLB_ACT_RELU6, STAGED>;
-    case PLB_ACT_LEAKY: return igemm_i8_tc_kernel<MODE, PLB_ACT_LEAKY, STAGED>;
-    default: return igemm_i8_tc_kernel<MODE, PLB_ACT_NONE, STAGED>;
+    case PLB_ACT_RELU: return igemm_i8_tc_kernel<MODE, PLB_ACT_RELU, STORE>;
+    case PLB_ACT_RELU6: return igemm_i8_tc_kernel<MODE, PLB_ACT_RELU6, STORE>;
+    case PLB_ACT_LEAKY: return igemm_i8_tc_kernel<MODE, PLB_ACT_LEAKY, STORE>;
+    default: return igemm_i8_tc_kernel<MODE, PLB_ACT_NONE, STORE>;
   }
 }
 
-template <bool STAGED>
+template <int STORE>
 IgemmKernel pick_mode(int mode, int act) {
   switch (mode) {
-    case OUT_F32: return pick_act<OUT_F32, STAGED>(act);
-    case OUT_I8: return pick_act<OUT_I8, STAGED>(act);
-    case OUT_ACC: return igemm_i8_tc_kernel<OUT_ACC, PLB_ACT_NONE, STAGED>;
-    default: return igemm_i8_tc_kernel<OUT_ADD_RELU, PLB_ACT_NONE, STAGED>;
+    case OUT_F32: return pick_act<OUT_F32, STORE>(act);
+    case OUT_I8: return pick_act<OUT_I8, STORE>(act);
+    case OUT_ACC: return igemm_i8_tc_kernel<OUT_ACC, PLB_ACT_NONE, STORE>;
+    // (a residual tensor is channels-last: no NCHW form)
+    default: return igemm_i8_tc_kernel<OUT_ADD_RELU, PLB_ACT_NONE, STORE == STORE_NCHW ? STORE_DIRECT : STORE>;
   }
 }
 
-IgemmKernel pick_kernel(int mode, int act, bool staged) {
-  return staged ? pick_mode<true>(mode, act) : pick_mode<false>(mode, act);
+IgemmKernel pick_kernel(int mode, int act, int store) {
+  switch (store) {
+    case STORE_STAGED: return pick_mode<STORE_STAGED>(mode, act);
+    case STORE_NCHW: return pick_mode<STORE_NCHW>(mode, act);
+    default: return pick_mode<STORE_DIRECT>(mode, act);
+  }
 }
 
 // ---------------------------------------------------------------- host side
@@ -1449,6 +1565,14 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
     bn = 64;
   else if (!dual && cout16 == 256 && bn == 256 && tiles_m <= 2 * ctx->sm_count)
     bn = 128;  // (with more tiles the wide tile wins again: 3x3 256 -> 256 on 14 x 14 at 512 images, 49 us against 57)
+  const bool nchw = p.y_nchw != 0;
+  if (nchw && p.out_mode == OUT_ADD_RELU) return fail(PLB_E_UNSUPPORTED, "NCHW output has no residual form");
+  if (nchw && cout16 > 256) {
+    // Any multiple of 32 will do as a tile width here (the staged epilogue needs powers of two): equal shares of the
+    // channels instead of full tiles and a nearly empty last one.
+    const int share = ((cout16 + (cout16 + bn - 1) / bn - 1) / ((cout16 + bn - 1) / bn) + 31) / 32 * 32;
+    if (share < bn) bn = share;
+  }
   bn = sw_or(sw_.bn, bn);
   if (dual && bn > 128) bn = 128;  // also after an override: two accumulators per tile must fit the 512 TMEM columns
   if (bn > cout16) bn = cout16;
@@ -1461,7 +1585,7 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
                       (p.out_mode == OUT_ADD_RELU && (p.y_f32 != nullptr || p.residual != nullptr || dual));
   const bool want_b = p.out_mode == OUT_I8 || (p.out_mode == OUT_ADD_RELU && p.y_i8 != nullptr);
   auto aligned16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  bool staged = sw_.staged != 0 && (bn == 32 || bn == 64 || bn == 128 || bn == 256);
+  bool staged = !nchw && sw_.staged != 0 && (bn == 32 || bn == 64 || bn == 128 || bn == 256);
   if (want_w && (p.ldy % 4 != 0)) staged = false;
   if (want_b && (p.ldy % 16 != 0)) staged = false;
   if (p.out_mode == OUT_ADD_RELU) {
@@ -1502,7 +1626,7 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
   }
   a.sb_off = a.staging_w_bytes + kEpilogueWarps * a.stage_b_warp;
   a.sb_cols = 0;
-  if (staged && p.out_mode != OUT_ACC && sw_.sb_smem != 0) {
+  if ((staged || nchw) && p.out_mode != OUT_ACC && sw_.sb_smem != 0) {
     const int cols = (p.cout + 31) / 32 * 32;  // the device arrays are readable up to the next multiple of 64 floats
     if (cols * 8 * (dual ? 2 : 1) <= 16 * 1024) a.sb_cols = cols;
   }
@@ -1523,7 +1647,7 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
   // once per tap.  Output tiles are 16 x 8 pixels, so images much smaller than that waste too
   // many accumulator rows.
   int tiles_m_eff = tiles_m;
-  if (p.im2col && a.taps > 1 && p.stride_h == 1 && p.stride_w == 1 && staged) {
+  if (p.im2col && a.taps > 1 && p.stride_h == 1 && p.stride_w == 1 && (staged || nchw)) {
     const int tx = (p.wo + 7) / 8, ty = (p.ho + 15) / 16;
     const int sw_px = 8 + (p.kw - 1) * p.dil_w, sh_px = 16 + (p.kh - 1) * p.dil_h;
     const double waste = static_cast<double>(tx) * 8 * ty * 16 / (static_cast<double>(p.wo) * p.ho);
@@ -1570,6 +1694,8 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
   a.out_mode = p.out_mode;
   a.ldy = p.ldy;
   a.y = p.y;
+  // (window tiles are rows of eight pixels, flat and im2col tiles run on across the rows and images of the batch)
+  a.nchw_words = nchw && (reinterpret_cast<uintptr_t>(p.y) & 3) == 0 && (a.slab ? p.wo % 4 == 0 : p.ho * p.wo % 4 == 0);
   a.scale = p.epi.scale; a.bias = p.epi.bias; a.act = p.epi.act; a.alpha = p.epi.alpha;
   a.acc_small = p.epi.acc_small && sw_.acc_small != 0;
   a.residual = p.residual; a.y_f32 = p.y_f32; a.y_i8 = p.y_i8;
@@ -1747,7 +1873,7 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
       return fail(PLB_E_INVALID, "tile of %d columns with %d accumulator buffers does not fit the 512 columns of tensor memory",
                   bn, a.acc_bufs);
   }
-  IgemmKernel kernel = pick_kernel(p.out_mode, p.epi.act, staged);
+  IgemmKernel kernel = pick_kernel(p.out_mode, p.epi.act, nchw ? STORE_NCHW : (staged ? STORE_STAGED : STORE_DIRECT));
   {
     // the attribute belongs to (function, device): remember which pairs have been configured
     std::lock_guard<std::mutex> lock(g_configure_mutex);
@@ -1770,7 +1896,7 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
 }  // namespace
 
 int igemm_tc_launch(plb_ctx* ctx, const IgemmProblem& p, IgemmPlanCache* cache) {
-  if (igemm_pair_wanted(ctx, p)) return igemm_pair_launch(ctx, p);
+  if (!p.y_nchw && igemm_pair_wanted(ctx, p)) return igemm_pair_launch(ctx, p);
   static const TcSwitches kDefaults;
   const TcSwitches& sw = p.sw ? *p.sw : kDefaults;
   const IgemmPlan* plan = nullptr;

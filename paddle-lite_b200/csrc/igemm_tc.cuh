@@ -59,6 +59,7 @@ struct IgemmProblem {
   int out_mode;
   void* y;           // OUT_F32 / OUT_I8 / OUT_ACC destination, row-major [m_total, ldy]
   int ldy;
+  int y_nchw;        // y is [batch, cout, ho, wo] instead (not with OUT_ADD_RELU; ldy unused)
   EpiParams epi;
   const float* residual;  // OUT_ADD_RELU
   float* y_f32;           // OUT_ADD_RELU, nullable

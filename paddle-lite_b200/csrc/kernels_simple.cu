@@ -95,6 +95,75 @@ __global__ void __launch_bounds__(kBlock)
   emit(o, m, co, acc);
 }
 
+// ------------------------------------------------------------------ fc of a few rows
+// With a handful of rows the layer is a pass over the filter (k * n bytes, from L2 or HBM) and a 128-row tensor-core
+// tile is nearly empty: its serial chain -- operand ring, MMA, tensor memory, staging -- took 6.0 us for one row of
+// 2048 x 1000 where the filter takes 0.3 us.  Here a warp owns one output feature: its lanes stride over K in 16-byte
+// pieces, dp4a against up to MR rows at once, one butterfly at the end.  The filter pieces of the first steps are
+// requested before the wait for the previous kernel (the filter is a layer constant), so their latency overlaps the
+// launch.
+constexpr int kFewRows = 8;
+template <int MR, bool VEC>
+__global__ void __launch_bounds__(kBlock)
+    fc_few_rows_kernel(const int8_t* __restrict__ x, const int8_t* __restrict__ w, const OutDev o, const int m, const int k,
+                       const int k_pad, const int n) {
+  constexpr int kAhead = 4;
+  const int lane = threadIdx.x & 31;
+  const int feature = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+  const bool live = feature < n;
+  const uint4* wr = reinterpret_cast<const uint4*>(w + static_cast<long>(live ? feature : 0) * k_pad);
+  const int pieces = k_pad / 16;
+  uint4 wv[kAhead];
+#pragma unroll
+  for (int j = 0; j < kAhead; ++j) {
+    const int p = j * 32 + lane;
+    wv[j] = live && p < pieces ? __ldg(wr + p) : make_uint4(0, 0, 0, 0);
+  }
+  pdl_sync_with_previous_kernel();
+  if (!live) return;
+  int acc[MR];
+#pragma unroll
+  for (int r = 0; r < MR; ++r) acc[r] = 0;
+  for (int p0 = 0; p0 < pieces; p0 += 32 * kAhead) {
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const int p = p0 + j * 32 + lane;
+      if (p >= pieces) break;
+      const uint4 v = wv[j];
+#pragma unroll
+      for (int r = 0; r < MR; ++r) {
+        if (r >= m) break;
+        const int8_t* xp = x + static_cast<long>(r) * k + 16 * p;
+        uint32_t xv[4];
+        if (VEC) {  // k is a multiple of 16: whole pieces
+          const uint4 t = __ldg(reinterpret_cast<const uint4*>(xp));
+          xv[0] = t.x; xv[1] = t.y; xv[2] = t.z; xv[3] = t.w;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) xv[e] = 16 * p + 4 * e < k ? __ldg(reinterpret_cast<const uint32_t*>(xp) + e) : 0u;
+        }
+        acc[r] = __dp4a(static_cast<int>(xv[0]), static_cast<int>(v.x), acc[r]);
+        acc[r] = __dp4a(static_cast<int>(xv[1]), static_cast<int>(v.y), acc[r]);
+        acc[r] = __dp4a(static_cast<int>(xv[2]), static_cast<int>(v.z), acc[r]);
+        acc[r] = __dp4a(static_cast<int>(xv[3]), static_cast<int>(v.w), acc[r]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const int p = p0 + (kAhead + j) * 32 + lane;
+      wv[j] = p < pieces ? __ldg(wr + p) : make_uint4(0, 0, 0, 0);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < MR; ++r)
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], s);
+  int mine = acc[0];
+#pragma unroll
+  for (int r = 1; r < MR; ++r) mine = lane == r ? acc[r] : mine;
+  if (lane < m && lane < MR) emit(o, lane, feature, mine);
+}
+
 // ------------------------------------------------------------------ depthwise convolution
 // One thread = one output pixel x 4 consecutive channels (one 32-bit load per tap).
 __global__ void __launch_bounds__(kBlock)
@@ -835,30 +904,45 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-// ---- fast int8 layout staging: 128-pixel x CT-channel tiles through shared memory, 128-bit
-// global accesses on the pixel-contiguous (NCHW) side, 4x4 byte transposes with prmt in registers.
-// The shared tile is [pixel][17 words] (CT <= 64 channels): odd pitch keeps the row-wise phase
-// conflict-free and the strided phase at four-way conflicts.
+// ---- int8 layout staging: tiles of 128-pixel strips x CT channels through shared memory, 16-byte accesses on both
+// sides, 4x4 byte transposes with prmt in registers.
 constexpr int kTilePix = 128;
-constexpr int kTilePitchW = 17;  // words per pixel row of the shared tile
+constexpr int kTilePitchW = 17;  // words per pixel row of the shared tile (the inverse kernel's)
 
-// x [n,c,hw] -> y [n,hw,cpad].  grid = (pixel strips, channel tiles, n); block = 256 threads =
-// 8 warps; a warp handles 4 channel quads x 8 segments of 16 pixels.  hw % 16 == 0.
+// 16 bytes starting at any byte address, from aligned 32-bit loads; words that lie wholly at or beyond `end`
+// are not read.
+__device__ __forceinline__ uint4 load16_unaligned(const uint8_t* p, const uint8_t* end) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~static_cast<uintptr_t>(3));
+  const uint32_t shift = static_cast<uint32_t>(a & 3) * 8;
+  uint32_t v[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) v[i] = reinterpret_cast<const uint8_t*>(w + i) < end ? __ldg(w + i) : 0u;
+  return make_uint4(__funnelshift_r(v[0], v[1], shift), __funnelshift_r(v[1], v[2], shift),
+                    __funnelshift_r(v[2], v[3], shift), __funnelshift_r(v[3], v[4], shift));
+}
+
+// x [n,c,hw] -> y [n,hw,cpad], cpad a multiple of CT (32 or 64), any hw.  grid = (groups of 128-pixel strips, channel
+// tiles, n); a warp reads 4 channel quads x 8 segments of 16 pixels.  VEC: x's rows start on 16-byte boundaries (planes
+// of a multiple of 16 pixels); else rows of any alignment are read as words and funnel-shifted (1.25 loads per word, a
+// byte-wise copy took 16 instructions per word: 122 images of 34 x 95 x 91 went from 150 us to the copy rate).
+// The shared tile is CT bytes per pixel; its 16-byte chunks are permuted inside each 128-byte line by the segment number,
+// which spreads the eight segments of a warp's word stores over the banks and leaves the 16-byte reads conflict-free.
+template <int CT, bool VEC>
 __global__ void __launch_bounds__(kBlock)
-    nchw_to_nhwc_i8_fast_kernel(const int8_t* __restrict__ x, int8_t* __restrict__ y, int c, int hw, int cpad,
-                                int ct) {
+    nchw_to_nhwc_i8_tile_kernel(const int8_t* __restrict__ x, int8_t* __restrict__ y, int c, int hw, int cpad, long total) {
   pdl_sync_with_previous_kernel();
-  extern __shared__ uint32_t tile_smem[];
-  const int cquads = ct / 4;                 // channel quads per tile (8 or 16)
-  const int warps_per_strip = cquads / 4;    // 2 or 4
-  const int strips = 8 / warps_per_strip;    // 128-pixel strips per block
+  constexpr int kWarpsPerStrip = CT / 16;          // 4 channel quads per warp
+  constexpr int kStrips = 8 / kWarpsPerStrip;      // 128-pixel strips per block
+  constexpr int kPixPerLine = 128 / CT;
+  __shared__ uint4 tile[kStrips * kTilePix * CT / 16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long n = blockIdx.z;
-  const int c0 = blockIdx.y * ct;
-  const int p_block = blockIdx.x * strips * kTilePix;
+  const int c0 = blockIdx.y * CT;
+  const int p_block = blockIdx.x * kStrips * kTilePix;
   {
-    const int strip = warp / warps_per_strip;
-    const int cq = (warp % warps_per_strip) * 4 + (lane >> 3);
+    const int strip = warp / kWarpsPerStrip;
+    const int cq = (warp % kWarpsPerStrip) * 4 + (lane >> 3);
     const int seg = lane & 7;
     const int p = p_block + strip * kTilePix + seg * 16;
     uint4 rows[4];
@@ -866,29 +950,42 @@ __global__ void __launch_bounds__(kBlock)
     for (int j = 0; j < 4; ++j) {
       const int ch = c0 + cq * 4 + j;
       rows[j] = make_uint4(0, 0, 0, 0);
-      if (ch < c && p < hw) rows[j] = __ldg(reinterpret_cast<const uint4*>(x + (n * c + ch) * static_cast<long>(hw) + p));
+      if (ch < c && p < hw) {
+        const int8_t* src = x + (n * c + ch) * static_cast<long>(hw) + p;
+        if (VEC) rows[j] = __ldg(reinterpret_cast<const uint4*>(src));
+        else rows[j] = load16_unaligned(reinterpret_cast<const uint8_t*>(src), reinterpret_cast<const uint8_t*>(x) + total);
+      }
     }
     const uint32_t* r0 = reinterpret_cast<const uint32_t*>(&rows[0]);
     const uint32_t* r1 = reinterpret_cast<const uint32_t*>(&rows[1]);
     const uint32_t* r2 = reinterpret_cast<const uint32_t*>(&rows[2]);
     const uint32_t* r3 = reinterpret_cast<const uint32_t*>(&rows[3]);
-    uint32_t* dst = tile_smem + (strip * kTilePix + seg * 16) * kTilePitchW + cq;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(tile) + (cq & 3);
+    const int line0 = (strip * kTilePix + seg * 16) / kPixPerLine;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       uint32_t w[4];
       transpose4x4(r0[g], r1[g], r2[g], r3[g], w);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) dst[(g * 4 + i) * kTilePitchW] = w[i];
+      for (int i = 0; i < 4; ++i) {
+        const int k = g * 4 + i;  // pixel of the segment
+        const int chunk = (k % kPixPerLine) * (CT / 16) + (cq >> 2);
+        dst[(line0 + k / kPixPerLine) * 32 + ((chunk ^ seg) << 2)] = w[i];
+      }
     }
   }
   __syncthreads();
-  const int words = strips * kTilePix * cquads;
-  for (int wi = threadIdx.x; wi < words; wi += kBlock) {
-    const int pix = wi / cquads, q = wi - pix * cquads;
+  constexpr int kChunks = kStrips * kTilePix * CT / 16;
+  int8_t* yn = y + n * hw * static_cast<long>(cpad) + c0;
+#pragma unroll
+  for (int i = threadIdx.x; i < kChunks; i += kBlock) {
+    const int pix = i / (CT / 16), k = i % (CT / 16);
     const int p = p_block + pix;
-    if (p < hw && c0 + q * 4 < cpad)
-      *reinterpret_cast<uint32_t*>(y + (n * hw + p) * static_cast<long>(cpad) + c0 + q * 4) =
-          tile_smem[pix * kTilePitchW + q];
+    if (p < hw) {
+      const int chunk = (pix % kPixPerLine) * (CT / 16) + k;
+      *reinterpret_cast<uint4*>(yn + p * static_cast<long>(cpad) + 16 * k) =
+          tile[(pix / kPixPerLine) * 8 + (chunk ^ ((pix >> 4) & 7))];
+    }
   }
 }
 
@@ -1200,19 +1297,6 @@ unsigned blocks_for(long total) { return static_cast<unsigned>((total + kBlock -
 // the NCHW-native tensor-core kernel and its output is copied back; both copies are small enough to be
 // served by the L2.
 
-// 16 bytes starting at any byte address, from aligned 32-bit loads; words that lie wholly at or beyond `end`
-// are not read.
-__device__ __forceinline__ uint4 load16_unaligned(const uint8_t* p, const uint8_t* end) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~static_cast<uintptr_t>(3));
-  const uint32_t shift = static_cast<uint32_t>(a & 3) * 8;
-  uint32_t v[5];
-#pragma unroll
-  for (int i = 0; i < 5; ++i) v[i] = reinterpret_cast<const uint8_t*>(w + i) < end ? __ldg(w + i) : 0u;
-  return make_uint4(__funnelshift_r(v[0], v[1], shift), __funnelshift_r(v[1], v[2], shift),
-                    __funnelshift_r(v[2], v[3], shift), __funnelshift_r(v[3], v[4], shift));
-}
-
 // src rows of `len` bytes back to back -> dst rows of `pitch` bytes (16-byte chunks; the tail of a row's last
 // chunk holds bytes of the following row, which the consumer's tensor map never reads as data).
 __global__ void __launch_bounds__(kBlock) pitch_rows_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
@@ -1321,6 +1405,26 @@ int conv_direct_launch(plb_ctx* ctx, const ConvGeom& g, const int8_t* x, const i
   if (total == 0) return PLB_OK;
   PLB_CUDA(launch_kernel(conv_direct_kernel, dim3(blocks_for(total)), dim3(kBlock), 0, ctx->stream, g, x, w_rsc, to_dev(out), total));
   PLB_CUDA(cudaGetLastError());
+  ctx->launches++;
+  return PLB_OK;
+}
+
+bool fc_few_rows_supported(int m, int k, const int8_t* x) {
+  return m <= kFewRows && k % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 3) == 0;
+}
+
+int fc_few_rows_launch(plb_ctx* ctx, const int8_t* x, int m, int k, const int8_t* w, int k_pad, int n, int mode, void* y,
+                       const EpiParams& epi) {
+  OutDev o;
+  memset(&o, 0, sizeof(o));
+  o.mode = mode; o.y = y; o.ldy = n;
+  o.scale = epi.scale; o.bias = epi.bias; o.act = epi.act; o.alpha = epi.alpha;
+  const bool vec = k % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  auto kern = m <= 1 ? (vec ? fc_few_rows_kernel<1, true> : fc_few_rows_kernel<1, false>)
+            : m <= 2 ? (vec ? fc_few_rows_kernel<2, true> : fc_few_rows_kernel<2, false>)
+            : m <= 4 ? (vec ? fc_few_rows_kernel<4, true> : fc_few_rows_kernel<4, false>)
+                     : (vec ? fc_few_rows_kernel<8, true> : fc_few_rows_kernel<8, false>);
+  PLB_CUDA(launch_kernel(kern, dim3((n + kBlock / 32 - 1) / (kBlock / 32)), dim3(kBlock), 0, ctx->stream, x, w, o, m, k, k_pad, n));
   ctx->launches++;
   return PLB_OK;
 }
@@ -1521,13 +1625,14 @@ int nchw_to_nhwc_i8_launch(plb_ctx* ctx, const int8_t* x, int8_t* y, int n, int 
   if (n == 0) return PLB_OK;
   if (cpad % 8 || cpad < c) return fail(PLB_E_INVALID, "cpad must be a multiple of 8 and >= c");
   const int hw = h * w;
-  if (hw % 16 == 0 && cpad % 32 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
-      (reinterpret_cast<uintptr_t>(y) & 3) == 0) {
+  if (cpad % 32 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
     const int ct = cpad % 64 == 0 ? 64 : 32;
     const int strips = 8 / (ct / 16);
+    const bool vec = hw % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
     dim3 fgrid((hw + strips * kTilePix - 1) / (strips * kTilePix), cpad / ct, n);
-    const size_t smem = static_cast<size_t>(strips) * kTilePix * kTilePitchW * 4;
-    PLB_CUDA(launch_kernel(nchw_to_nhwc_i8_fast_kernel, fgrid, dim3(kBlock), smem, ctx->stream, x, y, c, hw, cpad, ct));
+    auto kern = ct == 64 ? (vec ? nchw_to_nhwc_i8_tile_kernel<64, true> : nchw_to_nhwc_i8_tile_kernel<64, false>)
+                         : (vec ? nchw_to_nhwc_i8_tile_kernel<32, true> : nchw_to_nhwc_i8_tile_kernel<32, false>);
+    PLB_CUDA(launch_kernel(kern, fgrid, dim3(kBlock), 0, ctx->stream, x, y, c, hw, cpad, static_cast<long>(n) * c * hw));
     ctx->launches++;
     return PLB_OK;
   }

@@ -22,6 +22,7 @@ struct OutSpec {
   int mode;                   // OutMode of igemm_tc.cuh
   void* y;                    // [m_total, ldy]
   int ldy;
+  int y_nchw;                 // tensor-core path: y is [batch, cout, ho, wo]
   EpiParams epi;
   const float* residual;
   float* y_f32;
@@ -38,6 +39,11 @@ struct OutSpec {
 // Generic grouped convolution, NHWC in / NHWC out, one thread per output value.
 int conv_direct_launch(plb_ctx* ctx, const ConvGeom& g, const int8_t* x, const int8_t* w_rsc,
                        const OutSpec& out);
+// fc of a few rows: x [m, k] (k and the address multiples of 4), w [n, k_pad] (rows of whole 32-byte groups, zero past k),
+// y [m, n].
+bool fc_few_rows_supported(int m, int k, const int8_t* x);
+int fc_few_rows_launch(plb_ctx* ctx, const int8_t* x, int m, int k, const int8_t* w, int k_pad, int n, int mode, void* y,
+                       const EpiParams& epi);
 // Depthwise convolution, NHWC, channels multiple of 4 in storage; filter [kh*kw][c_stride].
 int dwconv_launch(plb_ctx* ctx, const ConvGeom& g, const int8_t* x, const int8_t* w_tc,
                   const OutSpec& out);

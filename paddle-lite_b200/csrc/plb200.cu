@@ -138,7 +138,6 @@ struct plb_fc {
   plb_ctx* ctx = nullptr;
   int k = 0, n = 0, k_pad = 0;
   int act = 0, out_dtype = 0;
-  bool tc = false;
   DeviceBuf wt;  // [n, k_pad]
   DeviceBuf scale_f32, bias_f32, scale_i8, bias_i8;
   float alpha_f32 = 0.f, alpha_i8 = 0.f;
@@ -458,7 +457,7 @@ int conv_core(plb_conv* c, const int8_t* x, int batch, const OutSpec& out) {
     p.m_total = batch * c->ho * c->wo;
     p.b = c->w.as<int8_t>();
     p.cout = d.cout;
-    p.out_mode = out.mode; p.y = out.y; p.ldy = out.ldy; p.epi = out.epi;
+    p.out_mode = out.mode; p.y = out.y; p.ldy = out.ldy; p.y_nchw = out.y_nchw; p.epi = out.epi;
     p.residual = out.residual; p.y_f32 = out.y_f32; p.y_i8 = out.y_i8;
     p.inv_next_scale = out.inv_next_scale;
     p.a2 = out.a2; p.b2 = out.b2; p.im2col2 = out.im2col2; p.h2 = out.h2; p.w2 = out.w2; p.cin_pad2 = out.cin_pad2;
@@ -512,14 +511,14 @@ bool nchw_native(const plb_conv* c, const int8_t* x, void* y, int batch, int mod
   p->out_mode = mode; p->y = y;
   p->bres_switch = c->sw.nchw_bres;
   if (p->hw % 16 != 0) {
-    // rows TMA cannot address: gather warps fill the operand tiles (igemm_nchw_gather.cu), several small images per tile
+    // Rows TMA cannot address: staged channels-last (one transposing pass in front of tiles that run across images and
+    // write NCHW themselves); the two variants below only when a switch asks for them.
+    if (c->sw.nchw != 1) return false;
+    // gather warps fill the operand tiles (igemm_nchw_gather.cu), several small images per tile
     if (c->sw.nchw_gather != 0 && igemm_nchw_gather_supported(c->ctx, *p, nullptr)) {
       p->x_pitch = -1;  // marks the gather kernel for the caller
       return true;
     }
-    // Images of fewer than 100 pixels would fill under half of a 128-pixel tile: the channels-last path, whose
-    // tiles run across images, serves them better.
-    if (p->hw < 100 && c->sw.nchw != 1) return false;
     // rows TMA cannot address: the caller stages x and y with rows a multiple of 16 bytes apart
     p->x_pitch = static_cast<int>(align_up(p->hw, 16));
     p->y_pitch = mode == OUT_I8 ? p->x_pitch : static_cast<int>(align_up(p->hw, 4));
@@ -567,6 +566,13 @@ int conv_run_nchw(plb_conv* c, const int8_t* x, void* y, int batch, int mode) {
   else
     rc = nchw_to_nhwc_i8_launch(ctx, x, xs, batch, d.cin, d.h, d.w, c->cin_pad);
   if (rc) return rc;
+  // The tensor-core kernel writes NCHW itself; the two-SM tiles (only when forced here) and the CUDA-core kernels write
+  // channels-last into the workspace.
+  if (c->kind == 0 && c->sw.pair != 1) {
+    OutSpec o = out_spec(c, mode, y);
+    o.y_nchw = 1;
+    return conv_core(c, xs, batch, o);
+  }
   OutSpec o = out_spec(c, mode, ys);
   if ((rc = conv_core(c, xs, batch, o))) return rc;
   return nhwc_to_nchw_launch(ctx, ys, y, batch, d.cout, c->ho, c->wo, mode == OUT_I8 ? 1 : 4);
@@ -813,8 +819,7 @@ int plb_fc_prepare(plb_ctx* ctx, int k, int n, int act, float act_alpha, float i
   f->out_dtype = out_dtype;
   f->sw = tc_switches_from_env();
   f->plans = igemm_plan_cache_create();
-  f->tc = (k % 32) == 0;
-  f->k_pad = f->tc ? k : static_cast<int>(align_up(k, 4));
+  f->k_pad = static_cast<int>(align_up(k, 32));
   std::vector<int8_t> wt(static_cast<size_t>(n) * f->k_pad, 0);  // [n][k]: K-major rows
   for (int kk = 0; kk < k; ++kk)
     for (int j = 0; j < n; ++j) wt[static_cast<size_t>(j) * f->k_pad + kk] = w_h[static_cast<size_t>(kk) * n + j];
@@ -853,18 +858,34 @@ static int fc_run_mode(plb_fc* f, const int8_t* x, void* y, int m, int mode) {
   }
   e.act = f->act;
   e.acc_small = f->acc_small ? 1 : 0;
-  if (f->tc && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+  if (f->k % 4 != 0) return fail(PLB_E_UNSUPPORTED, "fc with k %% 4 != 0 is not supported (k = %d)", f->k);
+  const int8_t* rows = x;
+  bool tc = true;
+  if (fc_few_rows_supported(m, f->k, x)) return fc_few_rows_launch(ctx, x, m, f->k, f->wt.as<int8_t>(), f->k_pad, f->n, mode, y, e);
+  if (f->k != f->k_pad || (reinterpret_cast<uintptr_t>(x) & 15) != 0) {
+    // Rows TMA cannot address: copied once into rows of k_pad bytes (the filter is zero there, so what the tail of a
+    // row holds does not matter).  One thread per output over the rows as they are took 670 us on 3200 x 1592 x 320.
+    const size_t need = static_cast<size_t>(m) * f->k_pad;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (need > ctx->ws_bytes) PLB_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
+    // (a workspace that cannot grow -- the caller's own, or during a capture -- leaves the CUDA-core kernel below)
+    tc = need <= ctx->ws_bytes || ((ctx->ws == nullptr || ctx->ws_owned) && capture == cudaStreamCaptureStatusNone);
+    if (tc) {
+      int rc = ctx->reserve(align_up(need, 256));
+      if (rc) return rc;
+      if ((rc = pitch_rows_i8_launch(ctx, x, ctx->ws, m, f->k, f->k_pad))) return rc;
+      rows = static_cast<const int8_t*>(ctx->ws);
+    }
+  }
+  if (tc) {
     IgemmProblem p;
     memset(&p, 0, sizeof(p));
-    p.a = x; p.im2col = 0; p.cin_pad = f->k; p.kh = p.kw = 1;
+    p.a = rows; p.im2col = 0; p.cin_pad = f->k_pad; p.kh = p.kw = 1;
     p.m_total = m; p.b = f->wt.as<int8_t>(); p.cout = f->n;
     p.out_mode = mode; p.y = y; p.ldy = f->n; p.epi = e;
     p.sw = &f->sw;
     return igemm_tc_launch(ctx, p, f->plans);
   }
-  // rows of x are not TMA-addressable: CUDA-core kernel on the same operands
-  if (f->k_pad != f->k)
-    return fail(PLB_E_UNSUPPORTED, "fc with k %% 4 != 0 is not supported (k = %d)", f->k);
   ConvGeom g;
   memset(&g, 0, sizeof(g));
   g.batch = m; g.cin = f->k; g.h = 1; g.w = 1; g.cin_stride = f->k; g.cout = f->n; g.kh = g.kw = 1;
