@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kBlock)
   const int feature = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
   const bool live = feature < n;
   const uint4* wr = reinterpret_cast<const uint4*>(w + static_cast<long>(live ? feature : 0) * k_pad);
-  const int pieces = k_pad / 16;
+  const int pieces = (k + 15) / 16;  // (not k_pad / 16: a whole piece past k would lie beyond the last row)
   uint4 wv[kAhead];
 #pragma unroll
   for (int j = 0; j < kAhead; ++j) {

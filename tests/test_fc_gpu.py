@@ -147,3 +147,26 @@ def test_random_fc_shapes(plb, ctx, m, k, n):
     ctx.sync()
     assert np.array_equal(y, y_ref)
     assert np.array_equal(q, q_ref)
+
+
+# rows at and around the filter pass for few rows (up to 8), and rows TMA addresses as they are (k % 16 == 0), after a copy
+# (k % 16 != 0) or through 32-byte groups; the last pieces of a row are whole, partial or missing
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 130])
+@pytest.mark.parametrize("k,n", [(4, 3), (16, 40), (48, 17), (524, 33), (1040, 100), (2064, 64), (2068, 48)])
+def test_fc_row_lengths(plb, ctx, m, k, n):
+    x, wq, ws, bias = fc_case(m * 3 + k + n, m, k, n)
+    acc_ref = O.fc_acc_i32(x, wq)
+    y_ref = O.epilogue(acc_ref, ws, 0.02, bias, O.ACT_LEAKY, 0.1)
+    out_s = float(max(np.abs(y_ref).max(), 1e-6) / 127)
+    q_ref = O.epilogue(acc_ref, ws, 0.02, bias, O.ACT_LEAKY, 0.1, out_scale=out_s)
+    fc = plb.Fc(ctx, wq, ws, 0.02, bias, O.ACT_LEAKY, 0.1)
+    fc8 = plb.Fc(ctx, wq, ws, 0.02, bias, O.ACT_LEAKY, 0.1, out_scale=out_s)
+    for offset in (0, 4):  # the second one: rows that start off the 16-byte grid
+        buf = torch.full((m * k + offset,), 77, dtype=torch.int8, device="cuda")
+        xd = buf[offset:].view(m, k)
+        xd.copy_(dev(x))
+        acc, y, q = fc.acc_i32(xd), fc.run(xd), fc8.run(xd)
+        ctx.sync()
+        assert np.array_equal(acc.cpu().numpy(), acc_ref)
+        assert np.array_equal(y.cpu().numpy(), y_ref)
+        assert np.array_equal(q.cpu().numpy(), q_ref)
