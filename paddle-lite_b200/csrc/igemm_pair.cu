@@ -513,8 +513,9 @@ int igemm_pair_launch(plb_ctx* ctx, const IgemmProblem& p) {
     if (r != CUDA_SUCCESS) return fail(PLB_E_CUDA, "cuTensorMapEncodeTiled(filter halves) failed: %d", (int)r);
   }
   if (!p.im2col) {
-    cuuint64_t dims[2] = {static_cast<cuuint64_t>(p.cin_pad), static_cast<cuuint64_t>(p.m_total)};
-    cuuint64_t strides[1] = {static_cast<cuuint64_t>(p.cin_pad)};
+    const cuuint64_t row = static_cast<cuuint64_t>(p.lda ? p.lda : p.cin_pad);
+    cuuint64_t dims[2] = {row, static_cast<cuuint64_t>(p.m_total)};
+    cuuint64_t strides[1] = {row};
     cuuint32_t box[2] = {static_cast<cuuint32_t>(a.kc), static_cast<cuuint32_t>(kRowsPerCta)};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = g_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(p.a), dims, strides, box, estr,

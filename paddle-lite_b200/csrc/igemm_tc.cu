@@ -1744,8 +1744,9 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(PLB_E_CUDA, "cuTensorMapEncodeTiled(input window) failed: %d", (int)r);
   } else if (!p.im2col) {
-    cuuint64_t dims[2] = {static_cast<cuuint64_t>(p.cin_pad), static_cast<cuuint64_t>(p.m_total)};
-    cuuint64_t strides[1] = {static_cast<cuuint64_t>(p.cin_pad)};
+    const cuuint64_t row = static_cast<cuuint64_t>(p.lda ? p.lda : p.cin_pad);
+    cuuint64_t dims[2] = {row, static_cast<cuuint64_t>(p.m_total)};
+    cuuint64_t strides[1] = {row};
     cuuint32_t box[2] = {static_cast<cuuint32_t>(a.kc), static_cast<cuuint32_t>(kTileM)};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = g_encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(p.a), dims,

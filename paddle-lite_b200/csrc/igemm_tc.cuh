@@ -45,10 +45,11 @@ TcSwitches tc_switches_from_env();
 // im2col view of an NHWC tensor; B is the filter repacked to [cout, taps * cin_pad].
 struct IgemmProblem {
   // A operand
-  const int8_t* a;   // flat: [m_total, cin_pad]; im2col: NHWC [batch, h, w, cin_pad]
+  const int8_t* a;   // flat: [m_total, lda]; im2col: NHWC [batch, h, w, cin_pad]
   int im2col;        // 0 flat, 1 im2col
   int batch, h, w;   // im2col only
-  int cin_pad;       // bytes per pixel / row, multiple of 32 (flat: multiple of 16)
+  int cin_pad;       // bytes per pixel / row, multiple of 32
+  int lda;           // flat: bytes from row to row, a multiple of 16; below cin_pad the missing bytes read as zero (0: cin_pad)
   int kh, kw, stride_h, stride_w, pad_t, pad_b, pad_l, pad_r, dil_h, dil_w;
   int ho, wo;
   int m_total;       // batch*ho*wo, or fc rows

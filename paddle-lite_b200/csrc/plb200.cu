@@ -498,6 +498,19 @@ OutSpec out_spec(const plb_conv* c, int mode, void* y) {
   return o;
 }
 
+// Whether a call that also has a path without scratch may take `need` bytes of the ctx workspace.  The caller's own
+// workspace must be large enough; the ctx's own is replaced by a larger one when it has to grow, so a call that is being
+// captured, whose graph would keep the address, stays away from it.
+bool may_stage(const plb_ctx* ctx, size_t need) {
+  if (ctx->ws != nullptr && !ctx->ws_owned) return need <= ctx->ws_bytes;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return capture == cudaStreamCaptureStatusNone;
+}
+
 // Unpadded stride-1 1x1 layers can run on the NCHW tensors as they are (igemm_nchw.cu): no staging passes.
 bool nchw_native(const plb_conv* c, const int8_t* x, void* y, int batch, int mode, NchwProblem* p) {
   const plb_conv_desc& d = c->d;
@@ -862,14 +875,13 @@ static int fc_run_mode(plb_fc* f, const int8_t* x, void* y, int m, int mode) {
   const int8_t* rows = x;
   bool tc = true;
   if (fc_few_rows_supported(m, f->k, x)) return fc_few_rows_launch(ctx, x, m, f->k, f->wt.as<int8_t>(), f->k_pad, f->n, mode, y, e);
-  if (f->k != f->k_pad || (reinterpret_cast<uintptr_t>(x) & 15) != 0) {
+  int lda = f->k;
+  if (f->k % 16 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0) {
     // Rows TMA cannot address: copied once into rows of k_pad bytes (the filter is zero there, so what the tail of a
     // row holds does not matter).  One thread per output over the rows as they are took 670 us on 3200 x 1592 x 320.
     const size_t need = static_cast<size_t>(m) * f->k_pad;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (need > ctx->ws_bytes) PLB_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
-    // (a workspace that cannot grow -- the caller's own, or during a capture -- leaves the CUDA-core kernel below)
-    tc = need <= ctx->ws_bytes || ((ctx->ws == nullptr || ctx->ws_owned) && capture == cudaStreamCaptureStatusNone);
+    lda = f->k_pad;
+    tc = may_stage(ctx, need);  // (else: the CUDA-core kernel below)
     if (tc) {
       int rc = ctx->reserve(align_up(need, 256));
       if (rc) return rc;
@@ -880,7 +892,7 @@ static int fc_run_mode(plb_fc* f, const int8_t* x, void* y, int m, int mode) {
   if (tc) {
     IgemmProblem p;
     memset(&p, 0, sizeof(p));
-    p.a = rows; p.im2col = 0; p.cin_pad = f->k_pad; p.kh = p.kw = 1;
+    p.a = rows; p.im2col = 0; p.cin_pad = f->k_pad; p.lda = lda; p.kh = p.kw = 1;
     p.m_total = m; p.b = f->wt.as<int8_t>(); p.cout = f->n;
     p.out_mode = mode; p.y = y; p.ldy = f->n; p.epi = e;
     p.sw = &f->sw;

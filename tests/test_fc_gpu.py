@@ -170,3 +170,41 @@ def test_fc_row_lengths(plb, ctx, m, k, n):
         assert np.array_equal(acc.cpu().numpy(), acc_ref)
         assert np.array_equal(y.cpu().numpy(), y_ref)
         assert np.array_equal(q.cpu().numpy(), q_ref)
+
+
+def test_fc_captured_call_keeps_no_scratch(plb):
+    """A graph of a layer whose rows are copied in an ordinary call (k % 16 != 0) stays good when the ctx workspace is
+    replaced by a larger one afterwards: the captured call does not use it."""
+    m, k, n = 40, 100, 64
+    x, wq, ws, bias = fc_case(5, m, k, n)
+    want = O.epilogue(O.fc_acc_i32(x, wq), ws, 0.02, bias, O.ACT_NONE, 0.0)
+    stream = torch.cuda.Stream()
+    own = plb.Context(0, stream=stream)
+    fc = plb.Fc(own, wq, ws, 0.02, bias)
+    xd, y = dev(x), torch.empty((m, n), device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        fc.run(xd, out=y)
+        own.sync()
+        size = own.workspace_size()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            fc.run(xd, out=y)
+        fc.run(dev(np.repeat(x, 50, axis=0)))
+        own.sync()
+        assert own.workspace_size() > size
+        y.zero_()
+        g.replay()
+        own.sync()
+    assert np.array_equal(y.cpu().numpy(), want)
+
+
+def test_fc_small_caller_workspace(plb):
+    """A workspace of the caller's that is too small for the copy of the rows: the layer runs without it."""
+    m, k, n = 40, 100, 64
+    x, wq, ws, bias = fc_case(6, m, k, n)
+    own = plb.Context(0)
+    own.set_workspace(torch.empty(1024, dtype=torch.uint8, device="cuda"))
+    y = plb.Fc(own, wq, ws, 0.02, bias).run(dev(x))
+    own.sync()
+    assert np.array_equal(y.cpu().numpy(), O.epilogue(O.fc_acc_i32(x, wq), ws, 0.02, bias, O.ACT_NONE, 0.0))
