@@ -525,13 +525,15 @@ bool nchw_native(const plb_conv* c, const int8_t* x, void* y, int batch, int mod
   p->bres_switch = c->sw.nchw_bres;
   if (p->hw % 16 != 0) {
     // Rows TMA cannot address: staged channels-last (one transposing pass in front of tiles that run across images and
-    // write NCHW themselves); the two variants below only when a switch asks for them.
-    if (c->sw.nchw != 1) return false;
+    // write NCHW themselves); the two variants below only when a switch asks for them or, the first of them, which needs
+    // no scratch, when there is none to be had.
+    if (c->sw.nchw != 1 && may_stage(c->ctx, plb_conv_workspace_bytes(c, batch))) return false;
     // gather warps fill the operand tiles (igemm_nchw_gather.cu), several small images per tile
     if (c->sw.nchw_gather != 0 && igemm_nchw_gather_supported(c->ctx, *p, nullptr)) {
       p->x_pitch = -1;  // marks the gather kernel for the caller
       return true;
     }
+    if (c->sw.nchw != 1) return false;
     // rows TMA cannot address: the caller stages x and y with rows a multiple of 16 bytes apart
     p->x_pitch = static_cast<int>(align_up(p->hw, 16));
     p->y_pitch = mode == OUT_I8 ? p->x_pitch : static_cast<int>(align_up(p->hw, 4));

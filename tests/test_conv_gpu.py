@@ -190,6 +190,70 @@ def test_nchw_images_tma_cannot_address(plb, ctx, case, gather, monkeypatch):
     assert ctx.nchw_gather_launch_count() == before_g + (3 if gather == "1" else 0)
 
 
+# (n, cin, h, w, cout, k, stride, pad, act): NCHW results written from the accumulators -- int8 words (planes or, in window
+# mode, rows of whole words) and single bytes, channel tiles of equal shares, ragged channels; rows at every byte alignment
+NCHW_EPILOGUE_CASES = [
+    (2, 64, 20, 20, 64, 3, 1, 1, 1),      # window mode needs more tiles than SMs: this is im2col, whole words
+    (40, 64, 48, 36, 48, 3, 1, 1, 2),     # window mode, rows of whole words, ragged last tile row, 48 channels
+    (40, 64, 47, 37, 64, 3, 1, 1, 3),     # window mode, odd rows
+    (3, 40, 9, 11, 300, 3, 1, 1, 3),      # 300 channels: equal tiles of 160 (or narrower), bytes
+    (2, 75, 13, 10, 272, 3, 2, 1, 1),     # strided, 35 pixels
+    (300, 32, 14, 14, 530, 1, 1, 0, 1),   # 1x1 on planes of whole words, three equal channel tiles
+    (5, 33, 7, 7, 17, 1, 1, 0, 0),        # fewer channels than a chunk, odd planes
+    (1, 64, 1, 1, 33, 1, 1, 0, 1),        # one pixel
+    (2, 16, 11, 9, 520, 5, 2, 2, 2),
+]
+
+
+@pytest.mark.parametrize("case", NCHW_EPILOGUE_CASES, ids=lambda c: "x".join(map(str, c[:7])))
+def test_nchw_results_from_the_accumulators(plb, ctx, case):
+    n, cin, h, w, cout, k, s, p, act = case
+    xq, in_s, wq, ws, bias = conv_case(sum(case), n, cin, h, w, cout, k)
+    run_case(plb, ctx, xq, in_s, wq, ws, bias, stride=(s, s), pads=(p, p, p, p), act=act,
+             alpha={2: 6.0, 3: 0.1}.get(act, 0.0))
+
+
+def test_nchw_staging_rows(plb, ctx):
+    """The staging pass reads rows of any byte alignment as words: planes of every residue of 16, offset buffers."""
+    rng = np.random.default_rng(8)
+    for n, c, hw, cpad in [(2, 5, 49, 32), (1, 34, 131, 64), (3, 64, 17, 64), (2, 33, 256, 96), (1, 1, 1, 32), (2, 70, 1023, 96)]:
+        x = rng.integers(-127, 128, (n, c, hw, 1), dtype=np.int8)
+        want = np.zeros((n, hw, 1, cpad), np.int8)
+        want[..., :c] = x.transpose(0, 2, 3, 1)
+        for offset in (0, 1, 7):
+            buf = torch.empty(x.size + offset, dtype=torch.int8, device="cuda")
+            xd = buf[offset:].view(x.shape)
+            xd.copy_(dev(x))
+            got = ctx.nchw_to_nhwc_i8(xd, cpad)
+            ctx.sync()
+            assert np.array_equal(got.cpu().numpy(), want), (n, c, hw, cpad, offset)
+
+
+def test_nchw_1x1_without_scratch(plb):
+    """1x1 layers on planes TMA cannot address need no workspace: a caller's that is too small, and captured calls."""
+    xq, in_s, wq, ws, bias = conv_case(12, 4, 64, 14, 14, 96, 1)
+    want = O.conv_int8(xq, wq, ws, in_s, bias, O.ACT_RELU)
+    x = dev(xq)
+    own = plb.Context(0)
+    own.set_workspace(torch.empty(1024, dtype=torch.uint8, device="cuda"))
+    y = plb.Conv(own, wq, ws, in_s, bias, in_hw=(14, 14), act=plb.ACT_RELU).run(x)
+    own.sync()
+    assert np.array_equal(y.cpu().numpy(), want)
+    stream = torch.cuda.Stream()
+    cap = plb.Context(0, stream=stream)
+    conv = plb.Conv(cap, wq, ws, in_s, bias, in_hw=(14, 14), act=plb.ACT_RELU)
+    y.zero_()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            conv.run(x, out=y)
+        assert cap.workspace_size() == 0
+        g.replay()
+        cap.sync()
+    assert np.array_equal(y.cpu().numpy(), want)
+
+
 def test_nchw_native_switch_off(plb, ctx, monkeypatch):
     monkeypatch.setenv("PLB_TC_NCHW", "0")
     xq, in_s, wq, ws, bias = conv_case(3, 2, 64, 16, 16, 64, 1)
