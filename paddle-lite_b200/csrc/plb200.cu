@@ -6,6 +6,7 @@
 #include <memory>
 #include <mutex>
 
+#include "dw_nchw.cuh"
 #include "fused_dwpw.cuh"
 #include "igemm_nchw.cuh"
 #include "igemm_tc.cuh"
@@ -431,6 +432,18 @@ int plb_softmax_f32(plb_ctx* ctx, const float* x, float* y, int rows, int cols) 
 
 namespace {
 
+ConvGeom conv_geom(const plb_conv* c, int batch) {
+  const plb_conv_desc& d = c->d;
+  ConvGeom g;
+  g.batch = batch; g.cin = d.cin; g.h = d.h; g.w = d.w; g.cin_stride = c->cin_pad;
+  g.cout = d.cout; g.kh = d.kh; g.kw = d.kw;
+  g.stride_h = d.stride_h; g.stride_w = d.stride_w; g.pad_t = d.pad_top; g.pad_l = d.pad_left;
+  g.dil_h = d.dil_h; g.dil_w = d.dil_w; g.groups = d.groups; g.ho = c->ho; g.wo = c->wo;
+  g.cg_pad = c->cg_pad;
+  g.dw_strip = c->sw.dw_strip;
+  return g;
+}
+
 // x is NHWC with channel stride conv->cin_pad.
 int conv_core(plb_conv* c, const int8_t* x, int batch, const OutSpec& out) {
   const plb_conv_desc& d = c->d;
@@ -465,13 +478,7 @@ int conv_core(plb_conv* c, const int8_t* x, int batch, const OutSpec& out) {
     p.sw = &c->sw;
     return igemm_tc_launch(ctx, p, c->plans);
   }
-  ConvGeom g;
-  g.batch = batch; g.cin = d.cin; g.h = d.h; g.w = d.w; g.cin_stride = c->cin_pad;
-  g.cout = d.cout; g.kh = d.kh; g.kw = d.kw;
-  g.stride_h = d.stride_h; g.stride_w = d.stride_w; g.pad_t = d.pad_top; g.pad_l = d.pad_left;
-  g.dil_h = d.dil_h; g.dil_w = d.dil_w; g.groups = d.groups; g.ho = c->ho; g.wo = c->wo;
-  g.cg_pad = c->cg_pad;
-  g.dw_strip = c->sw.dw_strip;
+  const ConvGeom g = conv_geom(c, batch);
   if (c->kind == 2) return dwconv_launch(ctx, g, x, c->w.as<int8_t>(), out);
   return conv_direct_launch(ctx, g, x, c->w.as<int8_t>(), out);
 }
@@ -568,6 +575,19 @@ int conv_run_nchw(plb_conv* c, const int8_t* x, void* y, int batch, int mode) {
       if ((rc = pitch_rows_i8_launch(ctx, x, base, static_cast<long>(batch) * d.cin, np.hw, np.x_pitch))) return rc;
       if ((rc = igemm_nchw_launch(ctx, np))) return rc;
       return unpitch_rows_launch(ctx, np.y, y, static_cast<long>(batch) * d.cout, np.hw, np.y_pitch, eb);
+    }
+  }
+  if (c->kind == 2 && c->sw.dw_strip < 0) {  // (a forced strip height means the channels-last kernel)
+    const ConvGeom g = conv_geom(c, batch);
+    if (dw_nchw_supported(g, mode)) {
+      // No scratch is needed here; where it can be had it is put in place all the same, so that the first call of a layer
+      // leaves a workspace of plb_conv_workspace_bytes() behind, whichever kernel its sizes take.
+      const size_t ws = plb_conv_workspace_bytes(c, batch);
+      if (ws > ctx->ws_bytes && may_stage(ctx, ws)) {
+        int rc = ctx->reserve(ws);
+        if (rc) return rc;
+      }
+      return dw_nchw_launch(ctx, g, x, c->w.as<int8_t>(), out_spec(c, mode, y));
     }
   }
   const size_t x_bytes = staged_input_bytes(c, batch);

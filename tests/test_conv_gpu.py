@@ -708,3 +708,39 @@ def test_im2col_role_loops_agree(plb, ctx, env, monkeypatch):
     q = conv8.run(dev(xq))
     ctx.sync()
     assert np.array_equal(q.cpu().numpy(), q_ref)
+
+
+# (n, c, h, w, k, stride, pads, act): whole planes in shared memory -- one to many planes per block at every byte alignment,
+# rows shorter than a group of four columns, one-pixel planes, pads wider than the filter's reach, several strips per plane
+DW_NCHW_CASES = [
+    (1, 1, 1, 1, 3, 1, (1, 1, 1, 1), 1),
+    (3, 700, 7, 7, 3, 1, (1, 1, 1, 1), 1),
+    (2, 333, 5, 3, 5, 1, (2, 2, 2, 2), 3),
+    (5, 61, 23, 29, 3, 2, (1, 1, 1, 1), 2),
+    (2, 37, 31, 18, 5, 2, (2, 2, 2, 2), 0),
+    (1, 6, 113, 111, 5, 1, (2, 2, 2, 2), 1),
+    (2, 3, 150, 160, 3, 1, (1, 1, 1, 1), 3),
+    (2, 16, 9, 11, 3, 1, (0, 2, 3, 1), 2),
+    (1, 20, 6, 6, 5, 2, (4, 4, 4, 4), 1),
+    (1, 2, 400, 300, 3, 1, (1, 1, 1, 1), 1),   # a plane that does not fit: the channels-last kernel
+]
+
+
+@pytest.mark.parametrize("case", DW_NCHW_CASES, ids=lambda c: "n%dc%dh%dw%dk%ds%d" % c[:6])
+def test_depthwise_nchw_planes(plb, ctx, case):
+    n, c, h, w, k, s, pads, act = case
+    xq, in_s, wq, ws, bias = conv_case(n + c * h + w * k, n, c, h, w, c, k, groups=c, w_std=0.3)
+    xq[0, 0, 0, 0] = -128
+    run_case(plb, ctx, xq, in_s, wq, ws, bias, stride=(s, s), pads=pads, groups=c, act=act,
+             alpha={2: 6.0, 3: 0.1}.get(act, 0.0))
+    # tensors that start anywhere
+    kw = dict(stride=(s, s), pads=pads, groups=c)
+    want = O.conv_int8(xq, wq, ws, in_s, bias, O.ACT_RELU, out_scale=0.05, **kw)
+    xd = torch.empty(xq.size + 5, dtype=torch.int8, device="cuda")[5:].view(xq.shape)
+    xd.copy_(dev(xq))
+    yd = torch.full((want.size + 14,), 99, dtype=torch.int8, device="cuda")
+    y = yd[7:-7].view(want.shape)
+    plb.Conv(ctx, wq, ws, in_s, bias, in_hw=(h, w), act=plb.ACT_RELU, out_scale=0.05, **kw).run(xd, out=y)
+    ctx.sync()
+    assert np.array_equal(y.cpu().numpy(), want)
+    assert (yd[:7] == 99).all() and (yd[-7:] == 99).all(), "bytes around the output were written"
