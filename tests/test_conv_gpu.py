@@ -744,3 +744,23 @@ def test_depthwise_nchw_planes(plb, ctx, case):
     ctx.sync()
     assert np.array_equal(y.cpu().numpy(), want)
     assert (yd[:7] == 99).all() and (yd[-7:] == 99).all(), "bytes around the output were written"
+
+
+@pytest.mark.parametrize("case", [(1, 16, 1, 1, 1, 1), (2, 48, 13, 10, 1, 1), (3, 32, 24, 18, 2, 3), (1, 64, 7, 33, 1, 2),
+                                  (40, 16, 9, 9, 2, 0), (2, 96, 34, 34, 1, 3)], ids=lambda c: "n%dc%dh%dw%ds%da%d" % c)
+def test_depthwise_5x5_channels_last(plb, ctx, case):
+    """5x5 layers on channels-last tensors: fewer rows and columns than a window, ragged last strips and column groups."""
+    n, c, h, w, s, act = case
+    xq, in_s, wq, ws, bias = conv_case(n * 7 + c + h, n, c, h, w, c, 5, groups=c, w_std=0.3)
+    kw = dict(stride=(s, s), pads=(2, 2, 2, 2), groups=c)
+    alpha = {2: 6.0, 3: 0.1}.get(act, 0.0)
+    acc = O.conv_acc_i32(xq, wq, **kw)
+    y_ref = O.epilogue(acc, ws, in_s, bias, act, alpha)
+    out_s = float(np.abs(y_ref).max() / 127)
+    q_ref = O.epilogue(acc, ws, in_s, bias, act, alpha, out_scale=out_s)
+    x = dev(np.ascontiguousarray(xq.transpose(0, 2, 3, 1)))
+    for scale, ref in ((None, y_ref), (out_s, q_ref)):
+        conv = plb.Conv(ctx, wq, ws, in_s, bias, in_hw=(h, w), act=act, alpha=alpha, out_scale=scale, **kw)
+        got = conv.run_nhwc(x).cpu().numpy().transpose(0, 3, 1, 2)
+        ctx.sync()
+        assert np.array_equal(got, ref)
