@@ -66,8 +66,8 @@ struct EpiParams {
   const float* bias;    // [C] folded bias(/out_s), zeros when absent
   int act;              // PLB_ACT_*
   float alpha;          // already divided by out_s where the reference does so
-  int acc_small = 0;    // 1: 128 * (largest sum of |w| over one output channel) < 2^22, so every accumulator is
-                        // below 2^22 in magnitude and converts to float exactly through the mantissa trick
+  int acc_small = 0;    // int8 results, 1: every |accumulator| < 2^22 (it converts to float exactly through the mantissa
+                        // trick) and every value in front of the rounding < 2^15 (it is clamped as a 16-bit integer)
   const float* h_scale = nullptr;  // host copies of scale / bias (or null): the one-launch first layer passes the
   const float* h_bias = nullptr;   // tables inside its kernel arguments
 };

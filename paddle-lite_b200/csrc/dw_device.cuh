@@ -74,5 +74,13 @@ __device__ __forceinline__ void dw_mac(int (&a)[4][4], const uint32_t (&win)[4][
     for (int c = 0; c < 4; ++c) a[ox][c] = __dp4a(static_cast<int>(win[ox][c]), static_cast<int>(wr[c]), a[ox][c]);
 }
 
+// The first filter row of an output starts from the magic bits itself: finished accumulators need no reset.
+__device__ __forceinline__ void dw_mac_first(int (&a)[4][4], const uint32_t (&win)[4][4], const uint32_t (&wr)[4]) {
+#pragma unroll
+  for (int ox = 0; ox < 4; ++ox)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) a[ox][c] = __dp4a(static_cast<int>(win[ox][c]), static_cast<int>(wr[c]), kDwMagic);
+}
+
 }  // namespace dw
 }  // namespace plb

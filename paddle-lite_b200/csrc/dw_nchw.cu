@@ -50,7 +50,7 @@ struct PlaneParams {
 
 // A strip of four output columns.  K x K filter, stride S.  `row` = byte offset (shared memory) of input row `ih`, first
 // column of the first window; rows outside the image and columns outside it (masks) read as zero.
-template <int K, int S, int MODE, int ACT>
+template <int K, int S, int MODE, int ACT, bool SMALL>
 __device__ __forceinline__ void strip4(const Args& a, const PlaneParams<K>& pp, const uint8_t* smem, int row, int ih, int iw,
                                        int rows, uint8_t* out, int ncols) {
   constexpr int kBytes = 3 * S + K;           // input bytes under four windows
@@ -110,7 +110,7 @@ __device__ __forceinline__ void strip4(const Args& a, const PlaneParams<K>& pp, 
         const int l = (p + kPeriod * K - r) / S % kLive;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          acc[l][j] = __dp4a(static_cast<int>(win[j]), static_cast<int>(wlo[r]), acc[l][j]);
+          acc[l][j] = __dp4a(static_cast<int>(win[j]), static_cast<int>(wlo[r]), r == 0 ? kDwMagic : acc[l][j]);
           if (K > 4) acc[l][j] = __dp4a(static_cast<int>(fifth[j]), static_cast<int>(whi[r]), acc[l][j]);
         }
       }
@@ -128,15 +128,13 @@ __device__ __forceinline__ void strip4(const Args& a, const PlaneParams<K>& pp, 
 #pragma unroll
           for (int j = 0; j < 4; ++j) v[j] = fmaf(__int_as_float(acc[l][j]) - tc::kRoundMagic, scale, bias);
           if (MODE == OUT_I8) {
-            uint32_t q[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) q[j] = __float_as_uint(tc::clamp_act<ACT>(v[j], a.alpha, ub) + tc::kRoundMagic);
+            const uint32_t q = tc::requant_pack4<ACT, SMALL>(make_float2(v[0], v[1]), make_float2(v[2], v[3]), a.alpha, ub);
             if (ncols >= 4 && (reinterpret_cast<uintptr_t>(out) & 3) == 0) {
-              *reinterpret_cast<uint32_t*>(out) = tc::pack_low_bytes(q[0], q[1], q[2], q[3]);
+              *reinterpret_cast<uint32_t*>(out) = q;
             } else {
 #pragma unroll
               for (int j = 0; j < 4; ++j)
-                if (j < ncols) out[j] = static_cast<uint8_t>(q[j]);
+                if (j < ncols) out[j] = static_cast<uint8_t>(q >> (8 * j));
             }
           } else {
 #pragma unroll
@@ -152,13 +150,11 @@ __device__ __forceinline__ void strip4(const Args& a, const PlaneParams<K>& pp, 
         }
         out += out_row;
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[l][j] = kDwMagic;
     }
   }
 }
 
-template <int K, int S, int MODE, int ACT>
+template <int K, int S, int MODE, int ACT, bool SMALL>
 __global__ void __launch_bounds__(kThreads) dw_nchw_kernel(const Args a) {
   extern __shared__ __align__(16) uint8_t smem[];
   pdl_sync_with_previous_kernel();
@@ -214,7 +210,7 @@ __global__ void __launch_bounds__(kThreads) dw_nchw_kernel(const Args a) {
     const int strip = in_plane / a.quads, quad = in_plane - strip * a.quads;
     const int oh = strip * a.strip, ow = quad * 4;
     const int ih = oh * S - a.pad_t, iw = ow * S - a.pad_l;
-    strip4<K, S, MODE, ACT>(a, params[plane], smem, kSlack + lead + plane * hw + ih * a.w_px + iw, ih, iw, min(a.strip, a.ho - oh),
+    strip4<K, S, MODE, ACT, SMALL>(a, params[plane], smem, kSlack + lead + plane * hw + ih * a.w_px + iw, ih, iw, min(a.strip, a.ho - oh),
                             out + (static_cast<long>(plane) * howo + oh * a.wo + ow) * EB, a.wo - ow);
   }
   __syncthreads();
@@ -232,23 +228,20 @@ __global__ void __launch_bounds__(kThreads) dw_nchw_kernel(const Args a) {
 }
 
 typedef void (*Kernel)(const Args);
-template <int K, int S>
-Kernel pick(int mode, int act) {
-  if (mode == OUT_ACC) return dw_nchw_kernel<K, S, OUT_ACC, PLB_ACT_NONE>;
-  if (mode == OUT_I8) {
-    switch (act) {
-      case PLB_ACT_RELU: return dw_nchw_kernel<K, S, OUT_I8, PLB_ACT_RELU>;
-      case PLB_ACT_RELU6: return dw_nchw_kernel<K, S, OUT_I8, PLB_ACT_RELU6>;
-      case PLB_ACT_LEAKY: return dw_nchw_kernel<K, S, OUT_I8, PLB_ACT_LEAKY>;
-      default: return dw_nchw_kernel<K, S, OUT_I8, PLB_ACT_NONE>;
-    }
-  }
+template <int K, int S, int MODE, bool SMALL>
+Kernel pick_act(int act) {
   switch (act) {
-    case PLB_ACT_RELU: return dw_nchw_kernel<K, S, OUT_F32, PLB_ACT_RELU>;
-    case PLB_ACT_RELU6: return dw_nchw_kernel<K, S, OUT_F32, PLB_ACT_RELU6>;
-    case PLB_ACT_LEAKY: return dw_nchw_kernel<K, S, OUT_F32, PLB_ACT_LEAKY>;
-    default: return dw_nchw_kernel<K, S, OUT_F32, PLB_ACT_NONE>;
+    case PLB_ACT_RELU: return dw_nchw_kernel<K, S, MODE, PLB_ACT_RELU, SMALL>;
+    case PLB_ACT_RELU6: return dw_nchw_kernel<K, S, MODE, PLB_ACT_RELU6, SMALL>;
+    case PLB_ACT_LEAKY: return dw_nchw_kernel<K, S, MODE, PLB_ACT_LEAKY, SMALL>;
+    default: return dw_nchw_kernel<K, S, MODE, PLB_ACT_NONE, SMALL>;
   }
+}
+template <int K, int S>
+Kernel pick(int mode, bool small, int act) {
+  if (mode == OUT_ACC) return dw_nchw_kernel<K, S, OUT_ACC, PLB_ACT_NONE, false>;
+  if (mode == OUT_F32) return pick_act<K, S, OUT_F32, false>(act);
+  return small ? pick_act<K, S, OUT_I8, true>(act) : pick_act<K, S, OUT_I8, false>(act);
 }
 
 // Shared memory of a block of n planes: {slack, input, slack} {parameters} {output}.
@@ -297,8 +290,9 @@ int dw_nchw_launch(plb_ctx* ctx, const ConvGeom& g, const int8_t* x, const int8_
   a.out_off = static_cast<int>(l.out_off);
   const long blocks = (a.planes + n - 1) / n;
   if (blocks > 0x7fffffffL) return fail(PLB_E_UNSUPPORTED, "depthwise: too many blocks");
-  Kernel k = g.kh == 3 ? (g.stride_h == 1 ? pick<3, 1>(out.mode, out.epi.act) : pick<3, 2>(out.mode, out.epi.act))
-                       : (g.stride_h == 1 ? pick<5, 1>(out.mode, out.epi.act) : pick<5, 2>(out.mode, out.epi.act));
+  const bool small = out.epi.acc_small != 0;
+  Kernel k = g.kh == 3 ? (g.stride_h == 1 ? pick<3, 1>(out.mode, small, out.epi.act) : pick<3, 2>(out.mode, small, out.epi.act))
+                       : (g.stride_h == 1 ? pick<5, 1>(out.mode, small, out.epi.act) : pick<5, 2>(out.mode, small, out.epi.act));
   PLB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBytes));
   PLB_CUDA(launch_kernel(k, dim3(static_cast<unsigned>(blocks)), dim3(kThreads), static_cast<size_t>(l.bytes), ctx->stream, a));
   ctx->launches++;

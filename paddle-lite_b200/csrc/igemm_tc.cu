@@ -78,7 +78,7 @@ struct IgemmArgs {
   const float* bias;
   int act;
   float alpha;
-  int acc_small;                       // every |accumulator| < 2^22 (proven from the filter by the host)
+  int acc_small;                       // EpiParams::acc_small
   int fast_window;                     // window tiles of a row-folded stem layer (shapes 4x1 / 2x1, two MMAs per tap): short role loops
   int fast_flat;                       // flat tiles without a shortcut GEMM: short producer loop
   int fast_im2col, cin_bytes;          // im2col tiles without a shortcut GEMM: short producer loop; cchunks * kc

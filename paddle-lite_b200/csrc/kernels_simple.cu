@@ -5,6 +5,7 @@
 
 #include "dw_device.cuh"
 #include "igemm_tc.cuh"
+#include "tc_device.cuh"
 #include <cstdlib>
 
 namespace plb {
@@ -394,36 +395,23 @@ DwKernel pick_dw_act(int act) {
 
 
 // fp32 work is done two channels at a time with the packed f32x2 instructions (same IEEE results per lane).
-template <int ACT, bool OUT_IS_I8>
-__device__ __forceinline__ void dw_emit_row(int (&a)[4][4], const float4 sc, const float4 bi, const float alpha,
+// SMALL: EpiParams::acc_small.
+template <int ACT, bool OUT_IS_I8, bool SMALL>
+__device__ __forceinline__ void dw_emit_row(const int (&a)[4][4], const float4 sc, const float4 bi, const float alpha,
                                             const float ub, void* __restrict__ y, const long yoff, const int ldy,
                                             const int ncols) {
-  const float2 magic = make_float2(12582912.f, 12582912.f), neg_magic = make_float2(-12582912.f, -12582912.f);
+  const float2 neg_magic = make_float2(-12582912.f, -12582912.f);
 #pragma unroll
   for (int ox = 0; ox < 4; ++ox) {
     const float2 v01 = __ffma2_rn(__fadd2_rn(make_float2(__int_as_float(a[ox][0]), __int_as_float(a[ox][1])), neg_magic),
                                   make_float2(sc.x, sc.y), make_float2(bi.x, bi.y));
     const float2 v23 = __ffma2_rn(__fadd2_rn(make_float2(__int_as_float(a[ox][2]), __int_as_float(a[ox][3])), neg_magic),
                                   make_float2(sc.z, sc.w), make_float2(bi.z, bi.w));
-    float v[4] = {v01.x, v01.y, v23.x, v23.y};
-#pragma unroll
-    for (int c = 0; c < 4; ++c) a[ox][c] = kDwMagic;
+    const float v[4] = {v01.x, v01.y, v23.x, v23.y};
     if (ox >= ncols) continue;
     if (OUT_IS_I8) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float t = v[c];
-        if (ACT == PLB_ACT_NONE) t = fminf(fmaxf(t, -127.f), 127.f);
-        else if (ACT == PLB_ACT_RELU) t = fminf(fmaxf(t, 0.f), 127.f);
-        else if (ACT == PLB_ACT_RELU6) t = fminf(fmaxf(t, 0.f), ub);
-        else { t = t <= 0.f ? alpha * t : t; t = fminf(fmaxf(t, -127.f), 127.f); }
-        v[c] = t;
-      }
-      // + 1.5*2^23 (after the clamp, where the add is exact): round to nearest even, result in the low byte
-      const float2 q01 = __fadd2_rn(make_float2(v[0], v[1]), magic), q23 = __fadd2_rn(make_float2(v[2], v[3]), magic);
       *reinterpret_cast<uint32_t*>(static_cast<int8_t*>(y) + yoff + static_cast<long>(ox) * ldy) =
-          __byte_perm(__byte_perm(__float_as_uint(q01.x), __float_as_uint(q01.y), 0x0040),
-                      __byte_perm(__float_as_uint(q23.x), __float_as_uint(q23.y), 0x0040), 0x5410);
+          tc::requant_pack4<ACT, SMALL>(v01, v23, alpha, ub);
     } else {
       *reinterpret_cast<float4*>(static_cast<float*>(y) + yoff + static_cast<long>(ox) * ldy) =
           make_float4(dw_act<ACT>(v[0], alpha), dw_act<ACT>(v[1], alpha), dw_act<ACT>(v[2], alpha),
@@ -434,7 +422,7 @@ __device__ __forceinline__ void dw_emit_row(int (&a)[4][4], const float4 sc, con
 
 constexpr int kDwBlock = 128;  // four blocks per SM at <= 128 registers: finer scheduling than two of 256
 
-template <int S, int ACT, bool OUT_IS_I8, int CS>
+template <int S, int ACT, bool OUT_IS_I8, int CS, bool SMALL>
 __global__ void __launch_bounds__(kDwBlock, 4)
     dwconv3x3_strip_kernel(const ConvGeom g, const int8_t* __restrict__ x, const int8_t* __restrict__ w,
                            const OutDev o, const int cquads, const int tiles_x, const int strip_rows) {
@@ -507,18 +495,13 @@ __global__ void __launch_bounds__(kDwBlock, 4)
       for (int P = 0; P < 3; ++P) {
         const int ir = iy + P;
         dw_make_win<1>(cur[P], win);
-        dw_mac(acc[P], win, wr[0]);
+        dw_mac_first(acc[P], win, wr[0]);
         dw_mac(acc[(P + 2) % 3], win, wr[1]);
         dw_mac(acc[(P + 1) % 3], win, wr[2]);
         const int oy = ir - 2;
         if (oy >= 0 && oy < rows) {
-          dw_emit_row<ACT, OUT_IS_I8>(acc[(P + 1) % 3], sc, bi, alpha, ub, o.y, yoff, ldy, ncols);
+          dw_emit_row<ACT, OUT_IS_I8, SMALL>(acc[(P + 1) % 3], sc, bi, alpha, ub, o.y, yoff, ldy, ncols);
           yoff += yrow;
-        } else {
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[(P + 1) % 3][a][c] = kDwMagic;
         }
       }
 #pragma unroll
@@ -553,17 +536,12 @@ __global__ void __launch_bounds__(kDwBlock, 4)
           xrow += row_step;
         }
         dw_make_win<2>(cur[0], win);
-        dw_mac(acc[P], win, wr[0]);
+        dw_mac_first(acc[P], win, wr[0]);
         dw_mac(acc[P ^ 1], win, wr[2]);
         const int oy = (ir >> 1) - 1;
         if (oy >= 0 && oy < rows) {
-          dw_emit_row<ACT, OUT_IS_I8>(acc[P ^ 1], sc, bi, alpha, ub, o.y, yoff, ldy, ncols);
+          dw_emit_row<ACT, OUT_IS_I8, SMALL>(acc[P ^ 1], sc, bi, alpha, ub, o.y, yoff, ldy, ncols);
           yoff += yrow;
-        } else {
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[P ^ 1][a][c] = kDwMagic;
         }
         dw_make_win<2>(cur[1], win);
         dw_mac(acc[P], win, wr[1]);
@@ -578,27 +556,28 @@ __global__ void __launch_bounds__(kDwBlock, 4)
 
 typedef void (*DwStripKernel)(const ConvGeom, const int8_t*, const int8_t*, const OutDev, const int, const int,
                               const int);
-template <int S, bool I8, int CS>
+template <int S, bool I8, int CS, bool SMALL>
 DwStripKernel pick_dw_strip_act(int act) {
   switch (act) {
-    case PLB_ACT_RELU: return dwconv3x3_strip_kernel<S, PLB_ACT_RELU, I8, CS>;
-    case PLB_ACT_RELU6: return dwconv3x3_strip_kernel<S, PLB_ACT_RELU6, I8, CS>;
-    case PLB_ACT_LEAKY: return dwconv3x3_strip_kernel<S, PLB_ACT_LEAKY, I8, CS>;
-    default: return dwconv3x3_strip_kernel<S, PLB_ACT_NONE, I8, CS>;
+    case PLB_ACT_RELU: return dwconv3x3_strip_kernel<S, PLB_ACT_RELU, I8, CS, SMALL>;
+    case PLB_ACT_RELU6: return dwconv3x3_strip_kernel<S, PLB_ACT_RELU6, I8, CS, SMALL>;
+    case PLB_ACT_LEAKY: return dwconv3x3_strip_kernel<S, PLB_ACT_LEAKY, I8, CS, SMALL>;
+    default: return dwconv3x3_strip_kernel<S, PLB_ACT_NONE, I8, CS, SMALL>;
   }
 }
 // int8 output with the usual channel counts as pixel pitch gets the compile-time-pitch variants
 template <int S>
-DwStripKernel pick_dw_strip(bool i8, int act, int pitch) {
-  if (!i8) return pick_dw_strip_act<S, false, 0>(act);
+DwStripKernel pick_dw_strip(bool i8, int act, int pitch, bool small) {
+  if (!i8) return pick_dw_strip_act<S, false, 0, false>(act);
+  if (!small) return pick_dw_strip_act<S, true, 0, false>(act);
   switch (pitch) {
-    case 32: return pick_dw_strip_act<S, true, 32>(act);
-    case 64: return pick_dw_strip_act<S, true, 64>(act);
-    case 128: return pick_dw_strip_act<S, true, 128>(act);
-    case 256: return pick_dw_strip_act<S, true, 256>(act);
-    case 512: return pick_dw_strip_act<S, true, 512>(act);
-    case 1024: return pick_dw_strip_act<S, true, 1024>(act);
-    default: return pick_dw_strip_act<S, true, 0>(act);
+    case 32: return pick_dw_strip_act<S, true, 32, true>(act);
+    case 64: return pick_dw_strip_act<S, true, 64, true>(act);
+    case 128: return pick_dw_strip_act<S, true, 128, true>(act);
+    case 256: return pick_dw_strip_act<S, true, 256, true>(act);
+    case 512: return pick_dw_strip_act<S, true, 512, true>(act);
+    case 1024: return pick_dw_strip_act<S, true, 1024, true>(act);
+    default: return pick_dw_strip_act<S, true, 0, true>(act);
   }
 }
 
@@ -608,7 +587,7 @@ DwStripKernel pick_dw_strip(bool i8, int act, int pitch) {
 // (80 of them at stride 1, which with the filter's 40 leaves three blocks per SM; the 160 dp4a of a row cover its loads,
 // which run one row ahead).  The kernel of one pixel per thread, which took these layers before, spends 50 loads on four
 // outputs: 16 channels on 29 x 22, 4 images: 6.7 -> 4.9 us.
-template <int S, int ACT, bool OUT_IS_I8>
+template <int S, int ACT, bool OUT_IS_I8, bool SMALL>
 __global__ void __launch_bounds__(kDwBlock, 3)
     dwconv5x5_strip_kernel(const ConvGeom g, const int8_t* __restrict__ x, const int8_t* __restrict__ w, const OutDev o,
                            const int cquads, const int tiles_x, const int strip_rows) {
@@ -694,7 +673,7 @@ __global__ void __launch_bounds__(kDwBlock, 3)
           const int l = (p + kPeriod * K - r) / S % kLive;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            acc[l][j][c] = __dp4a(static_cast<int>(win[j]), static_cast<int>(wlo[r][c]), acc[l][j][c]);
+            acc[l][j][c] = __dp4a(static_cast<int>(win[j]), static_cast<int>(wlo[r][c]), r == 0 ? kDwMagic : acc[l][j][c]);
             acc[l][j][c] = __dp4a(static_cast<int>(fifth[j]), static_cast<int>(whi[r][c]), acc[l][j][c]);
           }
         }
@@ -702,25 +681,24 @@ __global__ void __launch_bounds__(kDwBlock, 3)
       if ((p + kPeriod * K - (K - 1)) % S != 0) continue;
       const int l = (p + kPeriod * K - (K - 1)) / S % kLive;  // complete with this row
       if (i >= K - 1 && i < in_rows) {
-        dw_emit_row<ACT, OUT_IS_I8>(acc[l], sc, bi, o.alpha, ub, o.y, yoff, o.ldy, ncols);
+        dw_emit_row<ACT, OUT_IS_I8, SMALL>(acc[l], sc, bi, o.alpha, ub, o.y, yoff, o.ldy, ncols);
         yoff += yrow;
-      } else {
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) acc[l][a][c] = kDwMagic;
       }
     }
   }
 }
-template <int S, bool I8>
+template <int S, bool I8, bool SMALL>
 DwStripKernel pick_dw5(int act) {
   switch (act) {
-    case PLB_ACT_RELU: return dwconv5x5_strip_kernel<S, PLB_ACT_RELU, I8>;
-    case PLB_ACT_RELU6: return dwconv5x5_strip_kernel<S, PLB_ACT_RELU6, I8>;
-    case PLB_ACT_LEAKY: return dwconv5x5_strip_kernel<S, PLB_ACT_LEAKY, I8>;
-    default: return dwconv5x5_strip_kernel<S, PLB_ACT_NONE, I8>;
+    case PLB_ACT_RELU: return dwconv5x5_strip_kernel<S, PLB_ACT_RELU, I8, SMALL>;
+    case PLB_ACT_RELU6: return dwconv5x5_strip_kernel<S, PLB_ACT_RELU6, I8, SMALL>;
+    case PLB_ACT_LEAKY: return dwconv5x5_strip_kernel<S, PLB_ACT_LEAKY, I8, SMALL>;
+    default: return dwconv5x5_strip_kernel<S, PLB_ACT_NONE, I8, SMALL>;
   }
+}
+template <int S>
+DwStripKernel pick_dw5(bool i8, bool small, int act) {
+  return !i8 ? pick_dw5<S, false, false>(act) : small ? pick_dw5<S, true, true>(act) : pick_dw5<S, true, false>(act);
 }
 
 // ------------------------------------------------------------------ sparse 1x1 convolution
@@ -1570,9 +1548,8 @@ int dwconv_launch(plb_ctx* ctx, const ConvGeom& g, const int8_t* x, const int8_t
     }
     const int strips = (g.ho + strip - 1) / strip;
     if (strips <= 65535 && g.batch <= 65535 && g.batch > 0) {
-      const bool i8 = out.mode == OUT_I8;
-      DwStripKernel k = g.stride_h == 1 ? (i8 ? pick_dw5<1, true>(out.epi.act) : pick_dw5<1, false>(out.epi.act))
-                                        : (i8 ? pick_dw5<2, true>(out.epi.act) : pick_dw5<2, false>(out.epi.act));
+      const bool i8 = out.mode == OUT_I8, small = out.epi.acc_small != 0;
+      DwStripKernel k = g.stride_h == 1 ? pick_dw5<1>(i8, small, out.epi.act) : pick_dw5<2>(i8, small, out.epi.act);
       dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(strips), static_cast<unsigned>(g.batch));
       PLB_CUDA(launch_kernel(k, grid, dim3(kDwBlock), 0, ctx->stream, g, x, w_tc, to_dev(out), cq, tiles_x, strip));
       ctx->launches++;
@@ -1607,7 +1584,8 @@ int dwconv_launch(plb_ctx* ctx, const ConvGeom& g, const int8_t* x, const int8_t
       const int strips = (g.ho + strip - 1) / strip;
       if (strips > 65535 || g.batch > 65535) return fail(PLB_E_UNSUPPORTED, "depthwise 3x3: more than 65535 strips or images");
       const int pitch = g.cin_stride == static_cast<int>(out.ldy) ? g.cin_stride : 0;
-      DwStripKernel ks = g.stride_h == 1 ? pick_dw_strip<1>(i8, out.epi.act, pitch) : pick_dw_strip<2>(i8, out.epi.act, pitch);
+      DwStripKernel ks = g.stride_h == 1 ? pick_dw_strip<1>(i8, out.epi.act, pitch, out.epi.acc_small != 0)
+                                         : pick_dw_strip<2>(i8, out.epi.act, pitch, out.epi.acc_small != 0);
       dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(strips), static_cast<unsigned>(g.batch));
       PLB_CUDA(launch_kernel(ks, grid, dim3(kDwBlock), 0, ctx->stream, g, x, w_tc, to_dev(out), cq, tiles_x, strip));
       ctx->launches++;

@@ -87,6 +87,19 @@ Folded fold(int c, const float* wscale, int n_wscale, const float* bias, float i
   return f;
 }
 
+// Whether the requantiser may work in 16-bit integers (EpiParams::acc_small).  sum_abs = sum of |w| per output channel:
+// int8 inputs make no accumulator larger than 128 times that.  A comparison that meets a NaN or an infinity fails.
+bool requant_small(const std::vector<long>& sum_abs, const Folded& f, int act) {
+  if (act == PLB_ACT_RELU6 && !(f.alpha_i8 >= 0.f)) return false;  // (the minimum instruction ends in a maximum with zero)
+  const double slope = act == PLB_ACT_LEAKY ? std::max(1.0, std::fabs(static_cast<double>(f.alpha_i8))) : 1.0;
+  for (size_t i = 0; i < sum_abs.size(); ++i) {
+    const double acc = 128.0 * sum_abs[i];
+    const double v = acc * std::fabs(static_cast<double>(f.scale_i8[i])) + std::fabs(static_cast<double>(f.bias_i8[i]));
+    if (!(acc < 1 << 22) || !(v * slope < 32000.0)) return false;
+  }
+  return true;
+}
+
 }  // namespace
 }  // namespace plb
 
@@ -129,7 +142,7 @@ struct plb_conv {
   DeviceBuf scale_f32, bias_f32, scale_i8, bias_i8;
   std::vector<float> h_scale_i8, h_bias_i8;  // host copies of the int8-out tables (row-folded first layers only)
   float alpha_f32 = 0.f, alpha_i8 = 0.f;
-  bool acc_small = false;  // 128 * max over channels of sum |w| < 2^22: accumulators convert to float exactly by the mantissa trick
+  bool acc_small = false;  // requant_small() of the int8-out tables
   TcSwitches sw;           // tuning switches, read from the environment when the layer was prepared
   IgemmPlanCache* plans = nullptr;  // tile plans and tensor maps of the (batch, pointers) this layer has run on
   ~plb_conv() { igemm_plan_cache_destroy(plans); }
@@ -282,15 +295,14 @@ int plb_conv_prepare(plb_ctx* ctx, const plb_conv_desc* desc, const int8_t* filt
   const int cig = d.cin / d.groups;
   const bool depthwise = d.groups == d.cin && d.cin == d.cout;
   const int taps = d.kh * d.kw;
+  std::vector<long> sum_abs(d.cout);
   {
-    long worst = 0;
     const size_t per_channel = static_cast<size_t>(cig) * taps;
     for (int co = 0; co < d.cout; ++co) {
       long sum = 0;
       for (size_t i = 0; i < per_channel; ++i) sum += std::abs(static_cast<int>(filter_h[co * per_channel + i]));
-      worst = std::max(worst, sum);
+      sum_abs[co] = sum;
     }
-    c->acc_small = worst * 128 < (1L << 22);
   }
   std::vector<int8_t> packed, packed16;
   if (depthwise && d.impl != PLB_IMPL_TC) {
@@ -383,6 +395,7 @@ int plb_conv_prepare(plb_ctx* ctx, const plb_conv_desc* desc, const int8_t* filt
   }
   c->alpha_f32 = f.alpha_f32;
   c->alpha_i8 = f.alpha_i8;
+  c->acc_small = requant_small(sum_abs, f, d.act);
   *out = c.release();
   return PLB_OK;
 }
@@ -858,14 +871,13 @@ int plb_fc_prepare(plb_ctx* ctx, int k, int n, int act, float act_alpha, float i
   std::vector<int8_t> wt(static_cast<size_t>(n) * f->k_pad, 0);  // [n][k]: K-major rows
   for (int kk = 0; kk < k; ++kk)
     for (int j = 0; j < n; ++j) wt[static_cast<size_t>(j) * f->k_pad + kk] = w_h[static_cast<size_t>(kk) * n + j];
+  std::vector<long> sum_abs(n);
   {
-    long worst = 0;
     for (int j = 0; j < n; ++j) {
       long sum = 0;
       for (int kk = 0; kk < k; ++kk) sum += std::abs(static_cast<int>(wt[static_cast<size_t>(j) * f->k_pad + kk]));
-      worst = std::max(worst, sum);
+      sum_abs[j] = sum;
     }
-    f->acc_small = worst * 128 < (1L << 22);
   }
   int rc = f->wt.upload(wt.data(), wt.size());
   if (rc) return rc;
@@ -878,6 +890,7 @@ int plb_fc_prepare(plb_ctx* ctx, int k, int n, int act, float act_alpha, float i
   if ((rc = f->bias_i8.upload(fo.bias_i8.data(), cb))) return rc;
   f->alpha_f32 = fo.alpha_f32;
   f->alpha_i8 = fo.alpha_i8;
+  f->acc_small = requant_small(sum_abs, fo, act);
   *out = f.release();
   return PLB_OK;
 }
