@@ -11,6 +11,7 @@
 #include "igemm_nchw.cuh"
 #include "igemm_tc.cuh"
 #include "kernels_simple.cuh"
+#include "sparse_tmem.cuh"
 #include "stem_tc.cuh"
 
 namespace plb {
@@ -167,6 +168,8 @@ struct plb_sparse {
   int nnz = 0;
   DeviceBuf row_ptr, col, val, bias_raw;
   DeviceBuf col_val;  // fp32: {input channel, weight bits} per non-zero
+  DeviceBuf tmem_rows, tmem_batches;  // fp32: the non-zeros as sparse_tmem.cu walks them (empty: it cannot take this layer)
+  int tmem_pixels = 0;
   DeviceBuf grp_ptr, grp_idx, grp_w;  // int8: non-zeros in groups of four for the slab kernel
   DeviceBuf scale, bias;
   float alpha = 0.f;
@@ -1065,6 +1068,12 @@ int plb_sparse_prepare(plb_ctx* ctx, const plb_sparse_desc* desc, const void* no
       memcpy(&cv[2 * i + 1], &valf[i], 4);
     }
     if ((rc = s->col_val.upload(cv.data(), cv.size() * sizeof(int32_t)))) return rc;
+    SparseTmemLists lists;
+    if (sparse_tmem_build(d.cin, d.cout, static_cast<long>(d.h) * d.w, row_ptr, col, valf, bias_h, &lists)) {
+      s->tmem_pixels = lists.pixels;
+      if ((rc = s->tmem_rows.upload(lists.rows.data(), lists.rows.size() * sizeof(int4)))) return rc;
+      if ((rc = s->tmem_batches.upload(lists.batches.data(), lists.batches.size() * sizeof(int)))) return rc;
+    }
   }
   if (d.is_int8) {
     std::vector<int> gptr(d.cout + 1, 0);
@@ -1137,6 +1146,13 @@ int plb_sparse_run(plb_sparse* sp, const void* x, void* y, int batch) {
   if (sparse_slab_supported(g, x, y))
     return sparse_slab_launch(sp->ctx, g, static_cast<const int8_t*>(x), sp->grp_ptr.as<int>(), sp->grp_idx.p,
                               sp->grp_w.p, e, y);
+  if (sp->tmem_rows.p) {
+    SparseTmemProblem p;
+    p.batch = batch; p.cin = g.cin; p.cout = g.cout; p.hw = g.hw; p.pixels = sp->tmem_pixels; p.nnz = sp->nnz;
+    p.x = static_cast<const float*>(x); p.rows = sp->tmem_rows.p; p.batches = sp->tmem_batches.p;
+    p.act = e.act; p.alpha = e.alpha; p.y = static_cast<float*>(y);
+    if (sparse_tmem_better(p)) return sparse_tmem_launch(sp->ctx, p);
+  }
   return sparse_csr_launch(sp->ctx, g, x, sp->row_ptr.as<int>(), sp->col.as<int>(), sp->val.p, sp->col_val.p,
                            sp->bias_raw.as<float>(), e, y);
 }

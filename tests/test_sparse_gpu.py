@@ -77,6 +77,56 @@ def test_sparse_fp32(plb, ctx, cin, cout, side, batch, semi):
     assert_f32_close(y, y64, rel=1e-5, floor=float(np.abs(y64).max()))
 
 
+# fp32 walk over tensor memory: row lengths 0 and up to 20 of every remainder of a batch, chunks of channels with empty rows
+# in front, between and behind, pixel groups across images, teams that share a group, planes of whole 16-byte groups or not
+@pytest.mark.parametrize("cin,cout,h,w,batch", [(8, 23, 4, 4, 1), (128, 25, 5, 5, 7), (129, 30, 8, 4, 70), (300, 41, 3, 11, 5),
+                                                (64, 4, 1, 1, 3), (640, 9, 7, 7, 12), (32, 3, 40, 40, 60), (40, 70, 9, 7, 40)])
+@pytest.mark.parametrize("act,alpha", [(0, 0.0), (2, 1.5), (3, 0.1)])
+def test_sparse_fp32_row_lengths(plb, ctx, cin, cout, h, w, batch, act, alpha):
+    rng = np.random.default_rng(cin + cout)
+    wf = np.zeros((cout, cin), np.float32)
+    for oc in range(cout):
+        cols = rng.permutation(cin)[:min(cin, oc if oc < 21 else 3)]
+        if oc % 5 == 4:
+            cols = cols[cols >= min(cin - 1, 128)]
+        wf[oc, cols] = rng.standard_normal(len(cols))
+    x = rng.standard_normal((batch, cin, h, w)).astype(np.float32)
+    bias = rng.standard_normal(cout).astype(np.float32) if act else None
+    enc = O.sparse_encode(wf, h * w)
+    sp = plb.SparseConv(ctx, enc["nonzero_weights"], enc["oc_nonzeros"], enc["diffs"], enc["first_ic"], enc["flag_semi"],
+                        cin=cin, cout=cout, in_hw=(h, w), bias=bias, act=act, alpha=alpha)
+    y_ref = O.sparse_conv_f32(x, wf, bias if bias is not None else np.zeros(cout, np.float32), act, alpha)
+    for offset in (0, 1):  # the second one: tensors off the 16-byte grid
+        xd = torch.empty(x.size + offset, device="cuda")[offset:].view(x.shape)
+        xd.copy_(dev(x))
+        yd = torch.full((y_ref.size + offset,), 7.0, device="cuda")[offset:].view(y_ref.shape)
+        sp.run(xd, out=yd)
+        ctx.sync()
+        assert np.array_equal(yd.cpu().numpy(), y_ref)
+
+
+def test_sparse_fp32_special_values(plb, ctx):
+    """Only the non-zeros take part: infinities and NaN in a channel reach exactly the outputs that read it, and a sum of
+    negative zeros stays one."""
+    cin, cout, hw = 150, 12, 6
+    rng = np.random.default_rng(3)
+    wf = np.where(rng.random((cout, cin)) < 0.1, rng.standard_normal((cout, cin)), 0).astype(np.float32)
+    wf[3, :] = 0
+    x = rng.standard_normal((2, cin, hw, hw)).astype(np.float32)
+    x[0, 5], x[1, 140], x[0, 70, 2, 3] = np.inf, np.nan, -np.inf
+    bias = rng.standard_normal(cout).astype(np.float32)
+    bias[3] = -0.0
+    enc = O.sparse_encode(wf, hw * hw)
+    y = plb.SparseConv(ctx, enc["nonzero_weights"], enc["oc_nonzeros"], enc["diffs"], enc["first_ic"], enc["flag_semi"],
+                       cin=cin, cout=cout, in_hw=(hw, hw), bias=bias).run(dev(x)).cpu().numpy()
+    ctx.sync()
+    y_ref = O.sparse_conv_f32(x, wf, bias, O.ACT_NONE)
+    assert np.array_equal(np.isnan(y), np.isnan(y_ref)) and np.isnan(y_ref).any()
+    ok = ~np.isnan(y_ref)
+    assert np.array_equal(y[ok].view(np.int32), y_ref[ok].view(np.int32))
+    assert np.all(np.signbit(y[:, 3]))
+
+
 # the sparse_conv benchmark shapes: MobileNetV1 pointwise layers at batch 256, 80 % of the weights masked
 CONFIG5 = [(32, 64, 112), (128, 128, 56), (256, 256, 28), (512, 512, 14), (1024, 1024, 7)]
 
