@@ -548,15 +548,21 @@ bool nchw_native(const plb_conv* c, const int8_t* x, void* y, int batch, int mod
   p->bres_switch = c->sw.nchw_bres;
   if (p->hw % 16 != 0) {
     // Rows TMA cannot address: staged channels-last (one transposing pass in front of tiles that run across images and
-    // write NCHW themselves); the two variants below only when a switch asks for them or, the first of them, which needs
-    // no scratch, when there is none to be had.
-    if (c->sw.nchw != 1 && may_stage(c->ctx, plb_conv_workspace_bytes(c, batch))) return false;
-    // gather warps fill the operand tiles (igemm_nchw_gather.cu), several small images per tile
+    // write NCHW themselves), or gather warps fill the operand tiles (igemm_nchw_gather.cu, several small images per tile),
+    // which needs no scratch and no pass of its own.  Measured, gathered / staged: 512 -> 512 on 14 x 14, 256 images 43.5 /
+    // 37.7 us; 292 -> 96 on 25 x 25, 228 images, fp32 91 / 39; 64 -> 512 on 50 x 50, 32 images, fp32 65 / 47.  Rows of whole
+    // words keep the gather where the layer has few output channels for the staging pass to pay for (32 -> 32 on 90 x 90, 8
+    // images, fp32 8.7 / 12.6; 480 -> 32 on 63 x 84, 106 images 163 / 168; but 800 -> 64 on 18 x 18, 64 images 24.3 / 20.3)
+    // or few input channels and int8 results (64 -> 512 on 50 x 50, 32 images 32.2 / 35.6).
+    const bool few = p->hw % 4 == 0 && ((d.cout <= 64 && d.cin <= 512) || (mode == OUT_I8 && d.cin <= 64));
+    if (c->sw.nchw != 1 && !few && may_stage(c->ctx, plb_conv_workspace_bytes(c, batch))) return false;
     if (c->sw.nchw_gather != 0 && igemm_nchw_gather_supported(c->ctx, *p, nullptr)) {
       p->x_pitch = -1;  // marks the gather kernel for the caller
       return true;
     }
-    if (c->sw.nchw != 1) return false;
+    // (the same few channels where that kernel does not pay: rows re-pitched around the TMA kernel.  64 -> 800 on 34 x 34, 3
+    // images, int8: 10.1 us, staged 12.4; images below 100 pixels would fill under half of its 128-pixel tiles)
+    if (c->sw.nchw != 1 && (!few || p->hw < 100)) return false;
     // rows TMA cannot address: the caller stages x and y with rows a multiple of 16 bytes apart
     p->x_pitch = static_cast<int>(align_up(p->hw, 16));
     p->y_pitch = mode == OUT_I8 ? p->x_pitch : static_cast<int>(align_up(p->hw, 4));
