@@ -106,17 +106,53 @@ bool requant_small(const std::vector<long>& sum_abs, const Folded& f, int act) {
 
 using namespace plb;
 
+// Workspaces come from one memory pool per device: a cudaMalloc of the tens of megabytes that staging takes costs 0.5 - 8 ms
+// in the first call of every context, out of the pool some microseconds once the process has had one of that size.  The pool
+// keeps at most kPoolKeep bytes that no context uses, and none at all when the last context of the device is gone.  It orders
+// reuse between streams itself.
+static std::mutex g_pool_mutex;
+static cudaMemPool_t g_pool[64] = {nullptr};
+static int g_pool_users[64] = {0};
+constexpr unsigned long long kPoolKeep = 512ull << 20;
+
+static cudaError_t pool_alloc(int device, size_t bytes, cudaStream_t stream, void** out) {
+  if (device >= 64) return cudaMalloc(out, bytes);
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (!g_pool[device]) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = device;
+      cudaError_t e = cudaMemPoolCreate(&g_pool[device], &props);
+      if (e != cudaSuccess) return e;
+      unsigned long long keep = kPoolKeep;
+      e = cudaMemPoolSetAttribute(g_pool[device], cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) return e;
+    }
+    pool = g_pool[device];
+  }
+  return cudaMallocFromPoolAsync(out, bytes, pool, stream);
+}
+static void pool_user(int device, int change) {
+  if (device >= 64) return;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  g_pool_users[device] += change;
+  if (g_pool_users[device] == 0 && g_pool[device]) cudaMemPoolTrimTo(g_pool[device], 0);
+}
+
 int plb_ctx::reserve(size_t bytes) {
   if (bytes <= ws_bytes) return PLB_OK;
   if (!ws_owned && ws != nullptr)
     return fail(PLB_E_NOMEM, "caller-provided workspace of %zu bytes is too small (%zu needed)",
                 ws_bytes, bytes);
-  // growing: wait for work that may still use the old buffer
+  // growing: wait for work that may still use the old buffer (which also refuses to grow during a capture)
   PLB_CUDA(cudaStreamSynchronize(stream));
   if (ws) PLB_CUDA(cudaFree(ws));
   ws = nullptr;
   ws_bytes = 0;
-  cudaError_t e = cudaMalloc(&ws, bytes);
+  cudaError_t e = pool_alloc(device, bytes, stream, &ws);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(PLB_E_NOMEM, "cudaMalloc of %zu workspace bytes failed: %s", bytes,
@@ -209,6 +245,7 @@ int plb_ctx_create(int device, void* cuda_stream, plb_ctx** out) {
   PLB_CUDA(cudaMemset(c->d_status, 0, 2 * sizeof(int)));
   PLB_CUDA(cudaMallocHost(&c->h_status, 2 * sizeof(int)));
   c->h_status[0] = c->h_status[1] = 0;
+  pool_user(device, 1);
   *out = c.release();
   return PLB_OK;
 }
@@ -220,6 +257,7 @@ void plb_ctx_destroy(plb_ctx* ctx) {
   if (ctx->ws && ctx->ws_owned) cudaFree(ctx->ws);
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
+  pool_user(ctx->device, -1);
   delete ctx;
 }
 
