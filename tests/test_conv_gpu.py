@@ -764,3 +764,29 @@ def test_depthwise_5x5_channels_last(plb, ctx, case):
         got = conv.run_nhwc(x).cpu().numpy().transpose(0, 3, 1, 2)
         ctx.sync()
         assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("limit", [31000.0, 33000.0, 7e4, 130.0], ids=lambda v: "max%g" % v)
+@pytest.mark.parametrize("act,alpha", [(0, 0.0), (1, 0.0), (2, 6.0), (2, 0.3), (2, -3.0), (3, 0.1), (3, -1.0)])
+def test_requantiser_in_16_bits(plb, ctx, act, alpha, limit):
+    """Values in front of the rounding up to just below and above what the 16-bit clamp takes, many of them ties: 1x1, 3x3 and
+    depthwise layers in both layouts."""
+    rng = np.random.default_rng(23)
+    for groups, cin, k in ((1, 64, 1), (1, 32, 3), (64, 64, 3), (64, 64, 5)):
+        xq = rng.integers(-128, 128, (2, cin, 9, 12), dtype=np.int8)
+        xq[0, :, :5] = 127
+        wq = rng.integers(-127, 128, (64, cin // groups, k, k), dtype=np.int8)
+        wq[::2] = np.abs(wq[::2])
+        sums = np.abs(wq.astype(np.int64)).reshape(64, -1).sum(axis=1)
+        ws = (limit / (128.0 * sums)).astype(np.float32)
+        ws[5::7] = 0.5  # ties
+        ws = np.minimum(ws, np.float32(limit) / (128 * sums).astype(np.float32))
+        bias = np.where(np.arange(64) % 3 == 0, 0.5, 0.0).astype(np.float32)
+        kw = dict(stride=(1, 1), pads=(k // 2,) * 4, groups=groups)
+        want = O.epilogue(O.conv_acc_i32(xq, wq, **kw), ws, 1.0, bias, act, alpha, out_scale=1.0)
+        conv = plb.Conv(ctx, wq, ws, 1.0, bias, in_hw=(9, 12), act=act, alpha=alpha, out_scale=1.0, **kw)
+        got = conv.run(dev(xq))
+        got_cl = conv.run_nhwc(dev(np.ascontiguousarray(xq.transpose(0, 2, 3, 1))))
+        ctx.sync()
+        assert np.array_equal(got.cpu().numpy(), want)
+        assert np.array_equal(got_cl.cpu().numpy().transpose(0, 3, 1, 2), want)
