@@ -64,7 +64,8 @@ void plb_ctx_destroy(plb_ctx* ctx);
  * last call (the flag is cleared). */
 int plb_ctx_sync(plb_ctx* ctx);
 /* Optional: hand the ctx a caller-owned scratch buffer (layout staging for the NCHW entry
- * points).  Without it the ctx grows its own with cudaMalloc on demand.  Replaces the
+ * points).  Without it the ctx grows its own on demand, from a memory pool that the contexts of
+ * a device share (at most 512 MB of it unused, none when the last context is gone).  Replaces the
  * per-Run TargetMalloc of the im2col buffer (conv_compute.cc:306-310). */
 int plb_ctx_set_workspace(plb_ctx* ctx, void* dptr, size_t bytes);
 /* Bytes of scratch the NCHW entry points of this object need for `batch` images. */
