@@ -50,6 +50,7 @@ struct plb_ctx {
   void* ws = nullptr;           // layout-staging scratch
   size_t ws_bytes = 0;
   bool ws_owned = false;
+  void* ws_fence = nullptr;     // ordinary device allocation that lives as long as an owned ws (release_workspace())
   long launches = 0;
   long window_launches = 0;     // tensor-core convolutions that ran in window (slab) mode
   long pair_launches = 0;       // GEMMs that ran as two-SM tiles (cta_group::2)
@@ -58,6 +59,7 @@ struct plb_ctx {
   long nchw_gather_launches = 0;  // ... of which on images TMA cannot address (operand tiles filled by gather warps)
   long nchw_launches = 0;       // 1x1 convolutions that ran on NCHW tensors directly (no layout staging)
   int reserve(size_t bytes);    // make ws at least `bytes`
+  cudaError_t release_workspace();  // give an owned ws back, when nothing on the device uses it any more
 };
 
 // ---------------------------------------------------------------- epilogue description

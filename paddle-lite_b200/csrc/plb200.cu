@@ -108,13 +108,13 @@ using namespace plb;
 
 // Workspaces come from one memory pool per device: a cudaMalloc of the tens of megabytes that staging takes costs 0.5 - 8 ms
 // in the first call of every context, out of the pool some microseconds once the process has had one of that size.  The pool
-// keeps at most kPoolKeep bytes that no context uses, and none at all when the last context of the device is gone.  It orders
-// reuse between streams itself.
+// keeps at most kPoolKeep bytes that no context uses, and none at all when the last context of the device is gone.
 static std::mutex g_pool_mutex;
 static cudaMemPool_t g_pool[64] = {nullptr};
 static int g_pool_users[64] = {0};
 constexpr unsigned long long kPoolKeep = 512ull << 20;
 
+// Memory that every stream may use when this returns.
 static cudaError_t pool_alloc(int device, size_t bytes, cudaStream_t stream, void** out) {
   if (device >= 64) return cudaMalloc(out, bytes);
   cudaMemPool_t pool = nullptr;
@@ -125,15 +125,25 @@ static cudaError_t pool_alloc(int device, size_t bytes, cudaStream_t stream, voi
       props.allocType = cudaMemAllocationTypePinned;
       props.location.type = cudaMemLocationTypeDevice;
       props.location.id = device;
-      cudaError_t e = cudaMemPoolCreate(&g_pool[device], &props);
-      if (e != cudaSuccess) return e;
+      if (cudaMemPoolCreate(&g_pool[device], &props) != cudaSuccess) {  // a device without pools
+        cudaGetLastError();
+        g_pool[device] = nullptr;
+        return cudaMalloc(out, bytes);
+      }
       unsigned long long keep = kPoolKeep;
-      e = cudaMemPoolSetAttribute(g_pool[device], cudaMemPoolAttrReleaseThreshold, &keep);
-      if (e != cudaSuccess) return e;
+      cudaMemPoolSetAttribute(g_pool[device], cudaMemPoolAttrReleaseThreshold, &keep);
     }
     pool = g_pool[device];
   }
-  return cudaMallocFromPoolAsync(out, bytes, pool, stream);
+  cudaError_t e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
+  if (e == cudaErrorMemoryAllocation) {  // what the pool holds unused may be what is missing
+    cudaGetLastError();
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
+  }
+  if (e != cudaSuccess) return e;
+  // the allocation is an operation of `stream`; a captured graph that keeps the address may run on any other
+  return cudaStreamSynchronize(stream);
 }
 static void pool_user(int device, int change) {
   if (device >= 64) return;
@@ -142,20 +152,34 @@ static void pool_user(int device, int change) {
   if (g_pool_users[device] == 0 && g_pool[device]) cudaMemPoolTrimTo(g_pool[device], 0);
 }
 
+// A captured graph keeps the address of the workspace and may be running on any stream.  cudaFree of pool memory waits for
+// nothing, and the block's next owner would write under that graph; cudaFree of ordinary memory waits for the device, so the
+// fence goes first.  (cudaDeviceSynchronize would wait too, but it is refused while another thread captures a stream, and
+// breaks that capture.)
+cudaError_t plb_ctx::release_workspace() {
+  void *fence = ws_fence, *block = ws_owned ? ws : nullptr;
+  ws = ws_fence = nullptr;
+  ws_bytes = 0;
+  ws_owned = false;
+  cudaError_t e = fence ? cudaFree(fence) : cudaSuccess;
+  if (block && e == cudaSuccess) e = cudaFree(block);
+  return e;
+}
+
 int plb_ctx::reserve(size_t bytes) {
   if (bytes <= ws_bytes) return PLB_OK;
   if (!ws_owned && ws != nullptr)
     return fail(PLB_E_NOMEM, "caller-provided workspace of %zu bytes is too small (%zu needed)",
                 ws_bytes, bytes);
-  // growing: wait for work that may still use the old buffer (which also refuses to grow during a capture)
+  // growing: wait for this stream's work first (which refuses to grow during a capture)
   PLB_CUDA(cudaStreamSynchronize(stream));
-  if (ws) PLB_CUDA(cudaFree(ws));
-  ws = nullptr;
-  ws_bytes = 0;
-  cudaError_t e = pool_alloc(device, bytes, stream, &ws);
+  PLB_CUDA(release_workspace());
+  cudaError_t e = cudaMalloc(&ws_fence, 256);
+  if (e == cudaSuccess) e = pool_alloc(device, bytes, stream, &ws);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    return fail(PLB_E_NOMEM, "cudaMalloc of %zu workspace bytes failed: %s", bytes,
+    ws = nullptr;
+    return fail(PLB_E_NOMEM, "allocation of %zu workspace bytes failed: %s", bytes,
                 cudaGetErrorString(e));
   }
   ws_bytes = bytes;
@@ -254,7 +278,7 @@ void plb_ctx_destroy(plb_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
-  if (ctx->ws && ctx->ws_owned) cudaFree(ctx->ws);
+  ctx->release_workspace();
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   pool_user(ctx->device, -1);
@@ -286,7 +310,7 @@ int plb_ctx_set_workspace(plb_ctx* ctx, void* dptr, size_t bytes) {
   PLB_REQUIRE(ctx != nullptr, "ctx must not be null");
   PLB_REQUIRE((reinterpret_cast<uintptr_t>(dptr) & 255) == 0, "workspace must be 256-byte aligned");
   PLB_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (ctx->ws && ctx->ws_owned) PLB_CUDA(cudaFree(ctx->ws));
+  PLB_CUDA(ctx->release_workspace());
   ctx->ws = dptr;
   ctx->ws_bytes = dptr ? bytes : 0;
   ctx->ws_owned = false;

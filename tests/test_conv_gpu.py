@@ -790,3 +790,48 @@ def test_requantiser_in_16_bits(plb, ctx, act, alpha, limit):
         ctx.sync()
         assert np.array_equal(got.cpu().numpy(), want)
         assert np.array_equal(got_cl.cpu().numpy().transpose(0, 3, 1, 2), want)
+
+
+def test_workspace_growth_waits_for_the_device(plb):
+    """A captured graph keeps the workspace's address and may run on any stream: growing the workspace, taking the caller's
+    and destroying the context wait for it, so that nobody is given the memory under it."""
+    xq, in_s, wq, ws, bias = conv_case(41, 8, 32, 30, 30, 48, 3)
+    neg = np.negative(xq)
+    want = O.conv_int8(xq, wq, ws, in_s, bias, O.ACT_RELU, pads=(1, 1, 1, 1))
+    want_neg = O.conv_int8(neg, wq, ws, in_s, bias, O.ACT_RELU, pads=(1, 1, 1, 1))
+    x, big = dev(xq), dev(np.tile(neg, (4, 1, 1, 1)))
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for give_back in ("grow", "set", "destroy"):
+        a, b = plb.Context(0, stream=streams[0]), plb.Context(0, stream=streams[1])
+        conv = plb.Conv(a, wq, ws, in_s, bias, in_hw=(30, 30), pads=(1, 1, 1, 1), act=plb.ACT_RELU)
+        other = plb.Conv(b, wq, ws, in_s, bias, in_hw=(30, 30), pads=(1, 1, 1, 1), act=plb.ACT_RELU)
+        y, y_big, y_other = torch.zeros(want.shape, device="cuda"), *torch.zeros((2, 32) + want.shape[1:], device="cuda")
+        conv.run(x, out=y)
+        a.sync()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=streams[0]):
+            torch.cuda._sleep(40_000_000)  # some 20 ms, then the layer
+            conv.run(x, out=y)
+        y.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[2]):
+            g.replay()
+            done = torch.cuda.Event()
+            done.record()
+        if give_back == "grow":
+            conv.run(big, out=y_big)
+        elif give_back == "set":
+            a.set_workspace(torch.empty(1 << 20, dtype=torch.uint8, device="cuda"))
+        else:
+            a.close()
+        waited = done.query()
+        other.run(big, out=y_other)  # the pool's next block
+        torch.cuda.synchronize()
+        del g
+        a.close()
+        b.close()
+        assert waited, "the workspace was given back under a running graph (%s)" % give_back
+        assert np.array_equal(y.cpu().numpy(), want), give_back
+        assert np.array_equal(y_other.cpu().numpy()[24:], want_neg), give_back
+        if give_back == "grow":
+            assert np.array_equal(y_big.cpu().numpy()[24:], want_neg)
