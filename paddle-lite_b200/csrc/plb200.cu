@@ -663,16 +663,7 @@ int conv_run_nchw(plb_conv* c, const int8_t* x, void* y, int batch, int mode) {
   }
   if (c->kind == 2 && c->sw.dw_strip < 0) {  // (a forced strip height means the channels-last kernel)
     const ConvGeom g = conv_geom(c, batch);
-    if (dw_nchw_supported(g, mode)) {
-      // No scratch is needed here; where it can be had it is put in place all the same, so that the first call of a layer
-      // leaves a workspace of plb_conv_workspace_bytes() behind, whichever kernel its sizes take.
-      const size_t ws = plb_conv_workspace_bytes(c, batch);
-      if (ws > ctx->ws_bytes && may_stage(ctx, ws)) {
-        int rc = ctx->reserve(ws);
-        if (rc) return rc;
-      }
-      return dw_nchw_launch(ctx, g, x, c->w.as<int8_t>(), out_spec(c, mode, y));
-    }
+    if (dw_nchw_supported(g, mode)) return dw_nchw_launch(ctx, g, x, c->w.as<int8_t>(), out_spec(c, mode, y));
   }
   const size_t x_bytes = staged_input_bytes(c, batch);
   int rc = ctx->reserve(plb_conv_workspace_bytes(c, batch));
