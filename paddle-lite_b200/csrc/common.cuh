@@ -50,6 +50,7 @@ struct plb_ctx {
   void* ws = nullptr;           // layout-staging scratch
   size_t ws_bytes = 0;
   bool ws_owned = false;
+  bool ws_captured = false;     // a captured call keeps the address of an owned ws
   void* ws_fence = nullptr;     // ordinary device allocation that lives as long as an owned ws (release_workspace())
   long launches = 0;
   long window_launches = 0;     // tensor-core convolutions that ran in window (slab) mode

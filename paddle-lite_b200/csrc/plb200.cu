@@ -160,14 +160,24 @@ cudaError_t plb_ctx::release_workspace() {
   void *fence = ws_fence, *block = ws_owned ? ws : nullptr;
   ws = ws_fence = nullptr;
   ws_bytes = 0;
-  ws_owned = false;
+  ws_owned = ws_captured = false;
   cudaError_t e = fence ? cudaFree(fence) : cudaSuccess;
   if (block && e == cudaSuccess) e = cudaFree(block);
   return e;
 }
 
+static bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // (the legacy stream while another one is captured)
+  return true;
+}
+
 int plb_ctx::reserve(size_t bytes) {
-  if (bytes <= ws_bytes) return PLB_OK;
+  if (bytes <= ws_bytes) {
+    if (ws_owned && !ws_captured) ws_captured = capturing(stream);
+    return PLB_OK;
+  }
   if (!ws_owned && ws != nullptr)
     return fail(PLB_E_NOMEM, "caller-provided workspace of %zu bytes is too small (%zu needed)",
                 ws_bytes, bytes);
@@ -585,15 +595,11 @@ OutSpec out_spec(const plb_conv* c, int mode, void* y) {
 
 // Whether a call that also has a path without scratch may take `need` bytes of the ctx workspace.  The caller's own
 // workspace must be large enough; the ctx's own is replaced by a larger one when it has to grow, so a call that is being
-// captured, whose graph would keep the address, stays away from it.
+// captured, whose graph would keep the address, stays away from it, and so does one that would replace what a graph keeps.
 bool may_stage(const plb_ctx* ctx, size_t need) {
   if (ctx->ws != nullptr && !ctx->ws_owned) return need <= ctx->ws_bytes;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return capture == cudaStreamCaptureStatusNone;
+  if (ctx->ws_captured && need > ctx->ws_bytes) return false;
+  return !capturing(ctx->stream);
 }
 
 // Unpadded stride-1 1x1 layers can run on the NCHW tensors as they are (igemm_nchw.cu): no staging passes.

@@ -835,3 +835,42 @@ def test_workspace_growth_waits_for_the_device(plb):
         assert np.array_equal(y_other.cpu().numpy()[24:], want_neg), give_back
         if give_back == "grow":
             assert np.array_equal(y_big.cpu().numpy()[24:], want_neg)
+
+
+def test_workspace_of_a_graph_is_not_replaced_for_calls_that_need_none(plb):
+    """fc rows TMA cannot address, 1x1 layers on planes it cannot address and depthwise layers all have a path without
+    scratch: they do not replace a workspace whose address a captured 3x3 layer keeps."""
+    stream = torch.cuda.Stream()
+    own = plb.Context(0, stream=stream)
+    xq, in_s, wq, ws, bias = conv_case(43, 2, 32, 12, 12, 32, 3)
+    conv = plb.Conv(own, wq, ws, in_s, bias, in_hw=(12, 12), pads=(1, 1, 1, 1))
+    want = O.conv_int8(xq, wq, ws, in_s, bias, O.ACT_NONE, pads=(1, 1, 1, 1))
+    x, y = dev(xq), torch.zeros(want.shape, device="cuda")
+    x1, s1, w1, ws1, b1 = conv_case(44, 40, 128, 14, 14, 128, 1)
+    pw = plb.Conv(own, w1, ws1, s1, b1, in_hw=(14, 14))
+    xd, sd, wd, wsd, bd = conv_case(45, 8, 64, 30, 30, 64, 3, groups=64, w_std=0.3)
+    depthwise = plb.Conv(own, wd, wsd, sd, bd, in_hw=(30, 30), pads=(1, 1, 1, 1), groups=64)
+    rng = np.random.default_rng(46)
+    xf, wf = rng.integers(-127, 128, (9000, 100), dtype=np.int8), rng.integers(-127, 128, (100, 64), dtype=np.int8)
+    fc = plb.Fc(own, wf, np.full(64, 0.01, np.float32), 0.02, None)
+    conv.run(x, out=y)
+    own.sync()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        conv.run(x, out=y)
+    size = own.workspace_size()
+    got = [pw.run(dev(x1)), depthwise.run(dev(xd)), fc.run(dev(xf))]
+    own.sync()
+    kept = own.workspace_size() == size
+    if kept:  # (its address would be stale)
+        y.zero_()
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+    del g
+    assert kept, "the workspace that the graph keeps was replaced"
+    assert np.array_equal(y.cpu().numpy(), want)
+    assert np.array_equal(got[0].cpu().numpy(), O.conv_int8(x1, w1, ws1, s1, b1, O.ACT_NONE))
+    assert np.array_equal(got[1].cpu().numpy(), O.conv_int8(xd, wd, wsd, sd, bd, O.ACT_NONE, pads=(1, 1, 1, 1), groups=64))
+    assert np.array_equal(got[2].cpu().numpy(), O.epilogue(O.fc_acc_i32(xf, wf), np.full(64, 0.01, np.float32), 0.02, None, O.ACT_NONE, 0.0))
