@@ -1747,6 +1747,11 @@ int nchw_to_nhwc_i8_launch(plb_ctx* ctx, const int8_t* x, int8_t* y, int n, int 
   if (n == 0) return PLB_OK;
   if (cpad % 8 || cpad < c) return fail(PLB_E_INVALID, "cpad must be a multiple of 8 and >= c");
   const int hw = h * w;
+  constexpr int kMaxImages = 65535;  // of one launch: an image is a z coordinate of the grid
+  for (; n > kMaxImages; n -= kMaxImages, x += static_cast<long>(kMaxImages) * c * hw, y += static_cast<long>(kMaxImages) * hw * cpad) {
+    int rc = nchw_to_nhwc_i8_launch(ctx, x, y, kMaxImages, c, h, w, cpad);
+    if (rc) return rc;
+  }
   if (cpad % 32 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
     const int ct = cpad % 64 == 0 ? 64 : 32;
     const int strips = 8 / (ct / 16);

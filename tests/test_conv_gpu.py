@@ -229,6 +229,25 @@ def test_nchw_staging_rows(plb, ctx):
             assert np.array_equal(got.cpu().numpy(), want), (n, c, hw, cpad, offset)
 
 
+@pytest.mark.parametrize("cin,cout,k,act", [(16, 160, 1, 1), (40, 24, 3, 0)], ids=["1x1", "3x3"])
+def test_nchw_more_images_than_a_grid_dimension(plb, ctx, cin, cout, k, act):
+    """Staged layers of more than 65535 images: the first ones, those around the limit and the last ones."""
+    n, at = 70000, [0, 1, 65534, 65535, 65536, 69999]
+    xq, in_s, wq, ws, bias = conv_case(61, 50, cin, 3, 3, cout, k)
+    x = dev(xq).repeat(n // 50, 1, 1, 1)
+    pick = dev(np.negative(xq[:len(at)]))
+    x[at] = pick
+    conv = plb.Conv(ctx, wq, ws, in_s, bias, in_hw=(3, 3), pads=(k // 2,) * 4, act=act, out_scale=0.02)
+    y = conv.run(x)
+    ctx.sync()
+    want = O.conv_int8(np.negative(xq[:len(at)]), wq, ws, in_s, bias, act, pads=(k // 2,) * 4, out_scale=0.02)
+    assert np.array_equal(y[at].cpu().numpy(), want)
+    ref = O.conv_int8(xq, wq, ws, in_s, bias, act, pads=(k // 2,) * 4, out_scale=0.02)
+    same = (y.view(n // 50, 50, cout, 3, 3) == dev(ref)).flatten(2).all(dim=2).flatten()
+    same[at] = True
+    assert bool(same.all())
+
+
 def test_nchw_1x1_without_scratch(plb):
     """1x1 layers on planes TMA cannot address need no workspace: a caller's that is too small, and captured calls."""
     xq, in_s, wq, ws, bias = conv_case(12, 4, 64, 14, 14, 96, 1)
