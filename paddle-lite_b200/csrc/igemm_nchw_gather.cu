@@ -710,9 +710,18 @@ bool plan_gather(const plb_ctx* ctx, const NchwProblem& p, GatherPlan* plan, std
 
 }  // namespace
 
-bool igemm_nchw_gather_supported(const plb_ctx* ctx, const NchwProblem& p, std::string* why) {
+bool igemm_nchw_gather_supported(const plb_ctx* ctx, const NchwProblem& p, std::string* why, NchwGatherShape* shape) {
   GatherPlan plan;
-  return plan_gather(ctx, p, &plan, why);
+  if (!plan_gather(ctx, p, &plan, why)) return false;
+  if (shape) {
+    const GatherArgs& a = plan.a;
+    shape->resident = a.bres;
+    shape->bn = a.bn;
+    shape->ksteps = a.ksteps;
+    shape->channel_tiles = a.tiles_m;
+    shape->waves = ((a.bres ? a.num_ptiles : a.num_tiles) + ctx->sm_count - 1) / ctx->sm_count;
+  }
+  return true;
 }
 
 int igemm_nchw_gather_launch(plb_ctx* ctx, const NchwProblem& p) {

@@ -1517,6 +1517,31 @@ bool igemm_tc_supported(const IgemmProblem& p, std::string* why) {
 
 namespace {
 
+// Output channels per tile of the planner's choice.
+int channel_tile(int cout16, int tiles_m, int sm_count, bool dual, bool residual, bool nchw) {
+  int bn = cout16 < 256 ? cout16 : 256;
+  if (dual && bn > 128) bn = 128;  // two accumulators per tile and still two tiles in flight
+  // small problems: shrink the channel tile until the grid covers the SMs
+  // (the epilogue works in chunks of 32 columns, so a tile that is not the last one of its row of
+  // tiles must be a multiple of 32 wide: halve only down to such widths)
+  while (bn > 32 && tiles_m * ((cout16 + bn - 1) / bn) < sm_count && (bn / 2) % 32 == 0) bn /= 2;
+  // Measured per layer (ResNet-50, batch 128): a convolution that adds an fp32 residual and writes fp32 + int8 is
+  // bound by its epilogue's HBM traffic and runs best with narrow tiles (512 channels on 28 x 28: 81 us at 64
+  // columns, 87 at 128, 90 at 256); a layer of 256 output channels has a single 256-wide tile per row of pixels
+  // and loses to wave quantisation (196 tiles on 148 SMs: 10.6 us against 9.9 us at 128 columns).
+  if (!dual && residual && cout16 >= 512 && bn > 64)
+    bn = 64;
+  else if (!dual && cout16 == 256 && bn == 256 && tiles_m <= 2 * sm_count)
+    bn = 128;  // (with more tiles the wide tile wins again: 3x3 256 -> 256 on 14 x 14 at 512 images, 49 us against 57)
+  if (nchw && cout16 > 256) {
+    // Any multiple of 32 will do as a tile width here (the staged epilogue needs powers of two): equal shares of the
+    // channels instead of full tiles and a nearly empty last one.
+    const int share = ((cout16 + (cout16 + bn - 1) / bn - 1) / ((cout16 + bn - 1) / bn) + 31) / 32 * 32;
+    if (share < bn) bn = share;
+  }
+  return bn;
+}
+
 // Derives tile shapes, the shared-memory budget, the kernel instance and all tensor maps of one problem.
 int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, IgemmPlan* plan) {
   std::string why;
@@ -1550,29 +1575,10 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
   a.kh = p.im2col ? p.kh : 1;
   a.ksteps = a.taps * a.cchunks;
   const int cout16 = (p.cout + 15) / 16 * 16;
-  int bn = cout16 < 256 ? cout16 : 256;
-  if (dual && bn > 128) bn = 128;  // two accumulators per tile and still two tiles in flight
-  // small problems: shrink the channel tile until the grid covers the SMs
   const int tiles_m = (p.m_total + kTileM - 1) / kTileM;
-  // (the epilogue works in chunks of 32 columns, so a tile that is not the last one of its row of
-  // tiles must be a multiple of 32 wide: halve only down to such widths)
-  while (bn > 32 && tiles_m * ((cout16 + bn - 1) / bn) < ctx->sm_count && (bn / 2) % 32 == 0) bn /= 2;
-  // Measured per layer (ResNet-50, batch 128): a convolution that adds an fp32 residual and writes fp32 + int8 is
-  // bound by its epilogue's HBM traffic and runs best with narrow tiles (512 channels on 28 x 28: 81 us at 64
-  // columns, 87 at 128, 90 at 256); a layer of 256 output channels has a single 256-wide tile per row of pixels
-  // and loses to wave quantisation (196 tiles on 148 SMs: 10.6 us against 9.9 us at 128 columns).
-  if (!dual && p.out_mode == OUT_ADD_RELU && p.residual != nullptr && cout16 >= 512 && bn > 64)
-    bn = 64;
-  else if (!dual && cout16 == 256 && bn == 256 && tiles_m <= 2 * ctx->sm_count)
-    bn = 128;  // (with more tiles the wide tile wins again: 3x3 256 -> 256 on 14 x 14 at 512 images, 49 us against 57)
   const bool nchw = p.y_nchw != 0;
   if (nchw && p.out_mode == OUT_ADD_RELU) return fail(PLB_E_UNSUPPORTED, "NCHW output has no residual form");
-  if (nchw && cout16 > 256) {
-    // Any multiple of 32 will do as a tile width here (the staged epilogue needs powers of two): equal shares of the
-    // channels instead of full tiles and a nearly empty last one.
-    const int share = ((cout16 + (cout16 + bn - 1) / bn - 1) / ((cout16 + bn - 1) / bn) + 31) / 32 * 32;
-    if (share < bn) bn = share;
-  }
+  int bn = channel_tile(cout16, tiles_m, ctx->sm_count, dual, p.out_mode == OUT_ADD_RELU && p.residual != nullptr, nchw);
   bn = sw_or(sw_.bn, bn);
   if (dual && bn > 128) bn = 128;  // also after an override: two accumulators per tile must fit the 512 TMEM columns
   if (bn > cout16) bn = cout16;
@@ -1895,6 +1901,13 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
 }
 
 }  // namespace
+
+int igemm_tc_nchw_waves(const plb_ctx* ctx, int m_total, int cout, int* bn_out) {
+  const int cout16 = (cout + 15) / 16 * 16, tiles_m = (m_total + kTileM - 1) / kTileM;
+  const int bn = channel_tile(cout16, tiles_m, ctx->sm_count, false, false, true);
+  *bn_out = bn;
+  return static_cast<int>((static_cast<long>(tiles_m) * ((cout + bn - 1) / bn) + ctx->sm_count - 1) / ctx->sm_count);
+}
 
 int igemm_tc_launch(plb_ctx* ctx, const IgemmProblem& p, IgemmPlanCache* cache) {
   if (!p.y_nchw && igemm_pair_wanted(ctx, p)) return igemm_pair_launch(ctx, p);

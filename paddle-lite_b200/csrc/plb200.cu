@@ -602,43 +602,90 @@ bool may_stage(const plb_ctx* ctx, size_t need) {
   return !capturing(ctx->stream);
 }
 
+enum NchwPath { NCHW_STAGED, NCHW_TMA, NCHW_GATHERED, NCHW_PITCHED };
+
+// 1x1 layers on planes whose rows TMA cannot address (pixel counts that are not a multiple of 16) have three paths:
+//  staged    one transposing pass in front of channels-last tiles that run across images and write NCHW themselves: two
+//            launches, 7 us of host time;
+//  gathered  gather warps fill the operand tiles (igemm_nchw_gather.cu): one launch, no scratch, but a serial chain of
+//            gathers per tile, with single bytes where planes are not whole words;
+//  pitched   rows re-pitched around the TMA kernel and back: three launches.
+// The lines below are measured on 1300 layers (5 to 112 pixels a side, 16 to 1024 channels, 1 to 256 images), gathered or
+// pitched / staged in us, int8 results unless they say fp32.  Staged runs in whole waves of tiles: the second one costs as
+// much as the first, which is what the others win by on small layers.  Over all of them the choice is 0.7 % from the best of
+// the three; staging all of them is 3 % from it and up to 1.85 times as slow.
+NchwPath path_1x1_odd(const plb_ctx* ctx, const NchwProblem& p, bool can_gather, const NchwGatherShape& g) {
+  const long pixels = static_cast<long>(p.batch) * p.hw;
+  int staged_bn = 0;
+  const int staged_waves = igemm_tc_nchw_waves(ctx, p.batch * p.hw, p.cout, &staged_bn);
+  const bool words = p.hw % 4 == 0;
+  if (p.out_mode == OUT_I8) {
+    // one K chunk: 128 -> 256 on 34 x 34, 59 images 14.7 / 21.0, odd planes only where several fit a tile: 128 -> 231 on 5 x 5,
+    // 233 images 8.1 / 11.2, but 64 -> 344 on 69 x 69, 4 images 23.2 / 16.5
+    if (can_gather && g.ksteps == 1 && (words || (p.hw <= 48 && g.channel_tiles == 2))) return NCHW_GATHERED;
+    // a second wave of staged tiles and little to move three times: 672 -> 544 on 34 x 46, one image 12.2 / 16.8; 128 -> 64 on
+    // 50 x 50, 4 images 8.8 / 12.3; but 288 -> 35 on 53 x 53, 13 images (12 MB) 17.0 / 14.0; 31 -> 64 on 13 x 13, 58 images
+    // (narrow tiles, short K) 10.1 / 8.1
+    if (staged_waves > 1 && pixels * (p.cin + p.cout) < 11000000 && p.hw >= (words ? 150 : 240) &&
+        (p.cin_pad >= 128 || staged_waves * staged_bn >= 96) && (p.cin_pad >= 256 || pixels >= 2000))
+      return NCHW_PITCHED;
+    return NCHW_STAGED;
+  }
+  if (!can_gather) return NCHW_STAGED;  // (fp32: pitched lost 339 of 348 layers that differ)
+  bool gather;
+  const bool full = p.hw <= 256 || (p.hw + 255) / 256 * 1024l <= p.hw * 5l;  // tiles of 256 pixels waste less than a fifth
+  if (g.resident) {
+    // a single pixel tile per SM and few gathers: 160 -> 256 on 40 x 57, 16 images 14.1 / 19.1; 32 -> 508 on 42 x 66, 12 images
+    // 19.6 / 24.5; but 96 -> 320 on 17 x 17, 62 images 17.5 / 13.2; 32 -> 224 on 67 x 100, 21 images 43 / 34
+    gather = g.waves == 1 && g.channel_tiles <= 5 && p.cin_pad * g.channel_tiles <= (words ? 512 : 256);
+  } else if (staged_waves == 1) {
+    // 32 -> 160 on 6 x 6, 55 images 5.1 / 7.3; 64 -> 32 on 2500 pixels, 5 images 5.8 / 6.3; but 192 -> 309 on 132 pixels 9.1 / 5.8
+    // and 128 -> 128 on 10 x 10, 9 images (tiles of 32 channels cover the SMs) 7.3 / 5.8
+    gather = (p.cin_pad <= 128 && (g.bn <= 128 || pixels >= 8000) && (p.cin_pad <= 64 || staged_bn > 32)) ||
+             (p.cin_pad <= 64 && p.cout <= 64) || (p.cin_pad <= 192 && pixels >= 12000);
+  } else if (g.waves <= 2) {
+    // 64 -> 64 on 95 x 104, 2 images 6.1 / 11.4; 96 -> 128 on 4180 pixels, 3 images 8.8 / 12.3; but 672 -> 864 on 120 pixels,
+    // 36 images 33.8 / 16.3; one channel tile and many pixels, as below: 790 -> 128 on 22 x 22, 146 images 42 / 53
+    gather = g.waves * p.cin_pad <= 400 || (g.channel_tiles == 1 && full && pixels >= 60000);
+  } else {
+    // by throughput: 512 -> 64 on 106 x 106, 19 images 64 / 83; 96 -> 93 on 8652 pixels, 72 images 73 / 86; but 64 -> 32 on
+    // 4488 pixels, 133 images 43 / 36; 64 -> 67 on 3332 pixels, 55 images 26 / 20; 352 -> 160 on 78 x 78, 34 images 116 / 69;
+    // 704 -> 128 on 18 x 18, 151 images (tiles of 256 pixels, a third of them empty) 46 / 33
+    gather = g.channel_tiles == 1 && full && (p.cin_pad >= 128 || (p.cout > 48 && p.cin_pad >= 96) || pixels < 150000);
+  }
+  return gather ? NCHW_GATHERED : NCHW_STAGED;
+}
+
 // Unpadded stride-1 1x1 layers can run on the NCHW tensors as they are (igemm_nchw.cu): no staging passes.
-bool nchw_native(const plb_conv* c, const int8_t* x, void* y, int batch, int mode, NchwProblem* p) {
+NchwPath nchw_path(const plb_conv* c, const int8_t* x, void* y, int batch, int mode, NchwProblem* p) {
   const plb_conv_desc& d = c->d;
-  if (c->kind != 0 || c->fold || c->sw.nchw == 0) return false;
+  if (c->kind != 0 || c->fold || c->sw.nchw == 0) return NCHW_STAGED;
   if (!(d.kh == 1 && d.kw == 1 && d.stride_h == 1 && d.stride_w == 1 && d.pad_top == 0 && d.pad_bottom == 0 &&
         d.pad_left == 0 && d.pad_right == 0))
-    return false;
+    return NCHW_STAGED;
   memset(p, 0, sizeof(*p));
   p->x = x; p->w = c->w.as<int8_t>();
   p->batch = batch; p->cin = d.cin; p->cin_pad = c->cin_pad; p->cout = d.cout; p->hw = d.h * d.w;
   p->out_mode = mode; p->y = y;
   p->bres_switch = c->sw.nchw_bres;
-  if (p->hw % 16 != 0) {
-    // Rows TMA cannot address: staged channels-last (one transposing pass in front of tiles that run across images and
-    // write NCHW themselves), or gather warps fill the operand tiles (igemm_nchw_gather.cu, several small images per tile),
-    // which needs no scratch and no pass of its own.  Measured, gathered / staged: 512 -> 512 on 14 x 14, 256 images 43.5 /
-    // 37.7 us; 292 -> 96 on 25 x 25, 228 images, fp32 91 / 39; 64 -> 512 on 50 x 50, 32 images, fp32 65 / 47.  Rows of whole
-    // words keep the gather where the layer has few output channels for the staging pass to pay for (32 -> 32 on 90 x 90, 8
-    // images, fp32 8.7 / 12.6; 480 -> 32 on 63 x 84, 106 images 163 / 168; but 800 -> 64 on 18 x 18, 64 images 24.3 / 20.3)
-    // or few input channels and int8 results (64 -> 512 on 50 x 50, 32 images 32.2 / 35.6).
-    const bool few = p->hw % 4 == 0 && ((d.cout <= 64 && d.cin <= 512) || (mode == OUT_I8 && d.cin <= 64));
-    if (c->sw.nchw != 1 && !few && may_stage(c->ctx, plb_conv_workspace_bytes(c, batch))) return false;
-    if (c->sw.nchw_gather != 0 && igemm_nchw_gather_supported(c->ctx, *p, nullptr)) {
-      p->x_pitch = -1;  // marks the gather kernel for the caller
-      return true;
-    }
-    // (the same few channels where that kernel does not pay: rows re-pitched around the TMA kernel.  64 -> 800 on 34 x 34, 3
-    // images, int8: 10.1 us, staged 12.4; images below 100 pixels would fill under half of its 128-pixel tiles)
-    if (c->sw.nchw != 1 && (!few || p->hw < 100)) return false;
-    // rows TMA cannot address: the caller stages x and y with rows a multiple of 16 bytes apart
+  if (p->hw % 16 == 0) return igemm_nchw_supported(*p, nullptr) ? NCHW_TMA : NCHW_STAGED;
+  NchwGatherShape g = {};
+  const bool can_gather = c->sw.nchw_gather != 0 && igemm_nchw_gather_supported(c->ctx, *p, nullptr, &g);
+  NchwPath path;
+  if (c->sw.nchw == 1)
+    path = can_gather ? NCHW_GATHERED : NCHW_PITCHED;
+  else if (can_gather && !may_stage(c->ctx, plb_conv_workspace_bytes(c, batch)))
+    path = NCHW_GATHERED;  // (the one that needs no scratch)
+  else
+    path = path_1x1_odd(c->ctx, *p, can_gather, g);
+  if (path == NCHW_PITCHED) {
+    // the caller stages x and y with rows a multiple of 16 bytes apart and fills in the addresses
+    if (p->cin_pad % 32 != 0 || (reinterpret_cast<uintptr_t>(y) & 15) != 0) return NCHW_STAGED;
     p->x_pitch = static_cast<int>(align_up(p->hw, 16));
     p->y_pitch = mode == OUT_I8 ? p->x_pitch : static_cast<int>(align_up(p->hw, 4));
-    const bool aligned = (reinterpret_cast<uintptr_t>(y) & 15) == 0;
-    p->x = nullptr; p->y = nullptr;  // filled in by the caller
-    return p->cin_pad % 32 == 0 && aligned;
+    p->x = nullptr; p->y = nullptr;
   }
-  return igemm_nchw_supported(*p, nullptr);
+  return path;
 }
 
 int conv_run_nchw(plb_conv* c, const int8_t* x, void* y, int batch, int mode) {
@@ -647,13 +694,11 @@ int conv_run_nchw(plb_conv* c, const int8_t* x, void* y, int batch, int mode) {
   PLB_CUDA(cudaSetDevice(ctx->device));
   {
     NchwProblem np;
-    if (nchw_native(c, x, y, batch, mode, &np)) {
+    const NchwPath path = nchw_path(c, x, y, batch, mode, &np);
+    if (path != NCHW_STAGED) {
       np.epi = out_spec(c, mode, y).epi;
-      if (np.x_pitch < 0) {
-        np.x_pitch = 0;
-        return igemm_nchw_gather_launch(ctx, np);
-      }
-      if (np.x_pitch == 0) return igemm_nchw_launch(ctx, np);
+      if (path == NCHW_GATHERED) return igemm_nchw_gather_launch(ctx, np);
+      if (path == NCHW_TMA) return igemm_nchw_launch(ctx, np);
       // pixel counts that are not a multiple of 16: re-pitch the rows into the workspace, run, copy back
       const int eb = mode == OUT_I8 ? 1 : 4;
       const size_t xs_bytes = align_up(static_cast<size_t>(batch) * d.cin * np.x_pitch, 256);

@@ -213,6 +213,49 @@ def test_nchw_results_from_the_accumulators(plb, ctx, case):
              alpha={2: 6.0, 3: 0.1}.get(act, 0.0))
 
 
+# (n, cin, h, w, cout, int8 results, path): both sides of each line of the choice between the three paths of 1x1 layers on
+# planes TMA cannot address
+PATHS_1X1 = [
+    (12, 18, 42, 42, 160, True, "gathered"),    # one K chunk, planes of whole words
+    (12, 18, 43, 43, 160, True, "pitched"),     # ... odd planes
+    (233, 128, 5, 5, 231, True, "gathered"),    # ... small odd planes, several per tile
+    (1, 672, 34, 46, 544, True, "pitched"),     # two waves of staged tiles, few bytes
+    (4, 64, 69, 69, 344, True, "pitched"),
+    (58, 31, 13, 13, 64, True, "staged"),       # ... but small planes
+    (1, 96, 15, 17, 64, True, "staged"),        # one wave
+    (55, 32, 6, 6, 160, False, "gathered"),     # fp32, one wave
+    (1, 192, 11, 12, 309, False, "staged"),
+    (2, 64, 95, 104, 64, False, "gathered"),    # two waves, short chains of gathers
+    (2, 416, 52, 53, 128, False, "staged"),     # ... long ones
+    (127, 32, 5, 5, 238, False, "gathered"),    # pixel-resident order, one tile per SM
+    (62, 96, 17, 17, 320, False, "staged"),     # ... many gathers
+    (40, 32, 60, 67, 32, False, "staged"),      # many waves, few channels
+    (12, 128, 60, 67, 33, False, "gathered"),
+    (3, 64, 25, 25, 64, False, "staged"),       # odd planes
+]
+
+
+@pytest.mark.parametrize("case", PATHS_1X1, ids=lambda c: "x".join(map(str, c[:5])) + ("i8" if c[5] else "f32"))
+def test_nchw_1x1_paths(plb, ctx, case):
+    n, cin, h, w, cout, i8, path = case
+    xq, in_s, wq, ws, bias = conv_case(sum(case[:5]), n, cin, h, w, cout, 1)
+    want = O.conv_int8(xq, wq, ws, in_s, bias, O.ACT_RELU, out_scale=0.03 if i8 else None)
+    conv = plb.Conv(ctx, wq, ws, in_s, bias, in_hw=(h, w), act=plb.ACT_RELU, out_scale=0.03 if i8 else None)
+    before, before_g = ctx.nchw_launch_count(), ctx.nchw_gather_launch_count()
+    y = conv.run(dev(xq))
+    ctx.sync()
+    native, gathered = ctx.nchw_launch_count() - before, ctx.nchw_gather_launch_count() - before_g
+    assert np.array_equal(y.cpu().numpy(), want)
+    assert (native, gathered) == {"staged": (0, 0), "gathered": (1, 1), "pitched": (1, 0)}[path]
+    # tensors off every alignment that the faster paths ask for
+    xd = torch.empty(xq.size + 1, dtype=torch.int8, device="cuda")[1:].view(xq.shape)
+    xd.copy_(dev(xq))
+    yd = torch.zeros(want.size + 1, dtype=torch.int8 if i8 else torch.float32, device="cuda")[1:].view(want.shape)
+    conv.run(xd, out=yd)
+    ctx.sync()
+    assert np.array_equal(yd.cpu().numpy(), want)
+
+
 def test_nchw_staging_rows(plb, ctx):
     """The staging pass reads rows of any byte alignment as words: planes of every residue of 16, offset buffers."""
     rng = np.random.default_rng(8)
