@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kBlock)
   const long n = m / (static_cast<long>(g.wo) * g.ho);
   const int cog = g.cout / g.groups, cig = g.cin / g.groups;
   const int grp = co / cog;
-  const bool vec4 = (cig & 3) == 0 && (g.cin_stride & 3) == 0 && (g.cg_pad & 3) == 0;
+  const bool vec4 = (cig & 3) == 0 && (g.cin_stride & 3) == 0 && (g.cg_pad & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 3) == 0;
   int acc = 0;
   for (int r = 0; r < g.kh; ++r) {
     const int ih = oh * g.stride_h - g.pad_t + r * g.dil_h;

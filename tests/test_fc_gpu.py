@@ -208,3 +208,31 @@ def test_fc_small_caller_workspace(plb):
     y = plb.Fc(own, wq, ws, 0.02, bias).run(dev(x))
     own.sync()
     assert np.array_equal(y.cpu().numpy(), O.epilogue(O.fc_acc_i32(x, wq), ws, 0.02, bias, O.ACT_NONE, 0.0))
+
+
+@pytest.mark.parametrize("m", [3, 40])
+@pytest.mark.parametrize("offset", [1, 2, 4])
+def test_fc_rows_off_the_word_grid_without_scratch(plb, m, offset):
+    """Rows that start off the 4-byte grid where no copy can be made (captured calls, a caller's workspace that is too small)."""
+    k, n = 96, 33
+    x, wq, ws, bias = fc_case(7, m, k, n)
+    want = O.epilogue(O.fc_acc_i32(x, wq), ws, 0.02, bias, O.ACT_NONE, 0.0)
+    xd = torch.empty(m * k + offset, dtype=torch.int8, device="cuda")[offset:].view(m, k)
+    xd.copy_(dev(x))
+    small = plb.Context(0)
+    small.set_workspace(torch.empty(256, dtype=torch.uint8, device="cuda"))
+    y = plb.Fc(small, wq, ws, 0.02, bias).run(xd)
+    small.sync()
+    assert np.array_equal(y.cpu().numpy(), want)
+    stream = torch.cuda.Stream()
+    own = plb.Context(0, stream=stream)
+    fc = plb.Fc(own, wq, ws, 0.02, bias)
+    y.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        fc.run(xd, out=y)
+    g.replay()
+    torch.cuda.synchronize()
+    del g
+    assert np.array_equal(y.cpu().numpy(), want)
