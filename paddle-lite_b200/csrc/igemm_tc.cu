@@ -1902,9 +1902,9 @@ int igemm_tc_plan(plb_ctx* ctx, const IgemmProblem& p, const TcSwitches& sw_, Ig
 
 }  // namespace
 
-int igemm_tc_nchw_waves(const plb_ctx* ctx, int m_total, int cout, int* bn_out) {
+int igemm_tc_waves(const plb_ctx* ctx, int m_total, int cout, bool nchw, int* bn_out) {
   const int cout16 = (cout + 15) / 16 * 16, tiles_m = (m_total + kTileM - 1) / kTileM;
-  const int bn = channel_tile(cout16, tiles_m, ctx->sm_count, false, false, true);
+  const int bn = channel_tile(cout16, tiles_m, ctx->sm_count, false, false, nchw);
   *bn_out = bn;
   return static_cast<int>((static_cast<long>(tiles_m) * ((cout + bn - 1) / bn) + ctx->sm_count - 1) / ctx->sm_count);
 }

@@ -90,7 +90,7 @@ long igemm_plan_cache_hits(const IgemmPlanCache* c);
 bool igemm_tc_supported(const IgemmProblem& p, std::string* why);
 // Enqueue on ctx->stream.  Returns PLB_OK or an error code.
 int igemm_tc_launch(plb_ctx* ctx, const IgemmProblem& p, IgemmPlanCache* cache = nullptr);
-// Tiles per SM, rounded up, of a layer that writes NCHW, and the output channels of a tile.
-int igemm_tc_nchw_waves(const plb_ctx* ctx, int m_total, int cout, int* bn);
+// Tiles per SM, rounded up, of a layer without a residual, and the output channels of a tile.
+int igemm_tc_waves(const plb_ctx* ctx, int m_total, int cout, bool nchw, int* bn);
 
 }  // namespace plb

@@ -224,6 +224,7 @@ struct plb_fc {
   int k = 0, n = 0, k_pad = 0;
   int act = 0, out_dtype = 0;
   DeviceBuf wt;  // [n, k_pad]
+  DeviceBuf w_rows;  // k % 32 != 0: [n, k], for one thread per output
   DeviceBuf scale_f32, bias_f32, scale_i8, bias_i8;
   float alpha_f32 = 0.f, alpha_i8 = 0.f;
   bool acc_small = false;
@@ -617,7 +618,7 @@ enum NchwPath { NCHW_STAGED, NCHW_TMA, NCHW_GATHERED, NCHW_PITCHED };
 NchwPath path_1x1_odd(const plb_ctx* ctx, const NchwProblem& p, bool can_gather, const NchwGatherShape& g) {
   const long pixels = static_cast<long>(p.batch) * p.hw;
   int staged_bn = 0;
-  const int staged_waves = igemm_tc_nchw_waves(ctx, p.batch * p.hw, p.cout, &staged_bn);
+  const int staged_waves = igemm_tc_waves(ctx, p.batch * p.hw, p.cout, true, &staged_bn);
   const bool words = p.hw % 4 == 0;
   if (p.out_mode == OUT_I8) {
     // one K chunk: 128 -> 256 on 34 x 34, 59 images 14.7 / 21.0, odd planes only where several fit a tile: 128 -> 231 on 5 x 5,
@@ -994,6 +995,10 @@ int plb_fc_prepare(plb_ctx* ctx, int k, int n, int act, float act_alpha, float i
   }
   int rc = f->wt.upload(wt.data(), wt.size());
   if (rc) return rc;
+  if (f->k_pad != k) {
+    for (int j = 1; j < n; ++j) memmove(&wt[static_cast<size_t>(j) * k], &wt[static_cast<size_t>(j) * f->k_pad], k);
+    if ((rc = f->w_rows.upload(wt.data(), static_cast<size_t>(n) * k))) return rc;
+  }
   Folded fo = fold(n, wscale_h, n_wscale, bias_h, in_scale, out_dtype == PLB_OUT_I8 ? out_scale : 1.f,
                    act, act_alpha, 0);
   const size_t cb = sizeof(float) * n;
@@ -1008,6 +1013,35 @@ int plb_fc_prepare(plb_ctx* ctx, int k, int n, int act, float act_alpha, float i
   return PLB_OK;
 }
 
+enum FcPath { FC_FEW_ROWS, FC_DIRECT, FC_TENSOR };
+
+// The kernel of an fc call: the filter pass for few rows, one thread per output, or tensor-core tiles (behind a copy of the
+// rows where TMA cannot address them: `copy`).  Costs in us, fitted to 320 layers of 1 to 4000 rows, k 64 to 25088, n 10 to
+// 16384; all but a few are within 10 % (the direct kernel 30 %), and what the choice loses to the better kernel is 0.3 % over
+// the calls of few rows and 1.2 % over those with odd rows.  Measured, filter pass / tiles: 8 x 2048 x 1000 7.9 / 6.1;
+// 4 x 2048 x 1000 5.0 / 6.1; 8 x 4096 x 4096 15.4 / 16.6; 8 x 25088 x 64 72 / 30; 2 x 25088 x 64 21 / 30.  One thread per
+// output / copy and tiles: 185 x 108 x 110 4.2 / 18.6 (int8 rows that are not whole words leave byte by byte);
+// 71 x 1240 x 194 19 / 27; 514 x 116 x 58 4.8 / 7.0; but 103 x 316 x 518 16.2 / 8.7; 1105 x 428 x 1330 223 / 17.
+static FcPath fc_path(const plb_fc* f, const int8_t* x, int m, int mode, bool copy) {
+  const bool few = fc_few_rows_supported(m, f->k, x);
+  const bool direct = !few && (f->k % 32 != 0 || copy) && (reinterpret_cast<uintptr_t>(x) & 3) == 0;
+  if (copy && !may_stage(f->ctx, static_cast<size_t>(m) * f->k_pad)) return few ? FC_FEW_ROWS : FC_DIRECT;
+  const double k = f->k, n = f->n, mk = static_cast<double>(m) * k, mn = static_cast<double>(m) * n;
+  if (few) {
+    const double pass = 1.8 + 0.03 * m + 3.3e-4 * mk + 8e-5 * k + 9.5e-5 * n + 3.1e-5 * mn + 1e-8 * mk * n;
+    const double tiles = 3.4 + 1.07e-3 * k + 5.5e-7 * k * std::max(0.0, n - 600) + (copy ? 1 : 0);
+    return pass < tiles ? FC_FEW_ROWS : FC_TENSOR;
+  }
+  if (!direct) return FC_TENSOR;
+  int bn = 0;
+  const double waves = igemm_tc_waves(f->ctx, m, f->n, false, &bn);
+  // per column of a tile: single bytes, words, fp32 rows off the 16-byte grid, rows TMA can write
+  const double column = f->n % 4 != 0 ? (mode == OUT_I8 ? 0.091 : 0.07) : mode == OUT_I8 && f->n % 16 != 0 ? 0.036 : 0.02;
+  const double one_thread = 2.6 + 0.011 * k + 3.65e-7 * mk * n + 5.5e-6 * k * n;
+  const double tiles = 3.4 + (copy ? 1 + 1.3e-6 * mk : 0) + waves * (bn * column + 1.8e-3 * k) + 9e-7 * mn;
+  return one_thread < tiles ? FC_DIRECT : FC_TENSOR;
+}
+
 static int fc_run_mode(plb_fc* f, const int8_t* x, void* y, int m, int mode) {
   plb_ctx* ctx = f->ctx;
   PLB_CUDA(cudaSetDevice(ctx->device));
@@ -1020,24 +1054,21 @@ static int fc_run_mode(plb_fc* f, const int8_t* x, void* y, int m, int mode) {
   e.act = f->act;
   e.acc_small = f->acc_small ? 1 : 0;
   if (f->k % 4 != 0) return fail(PLB_E_UNSUPPORTED, "fc with k %% 4 != 0 is not supported (k = %d)", f->k);
-  const int8_t* rows = x;
-  bool tc = true;
-  if (fc_few_rows_supported(m, f->k, x)) return fc_few_rows_launch(ctx, x, m, f->k, f->wt.as<int8_t>(), f->k_pad, f->n, mode, y, e);
-  int lda = f->k;
-  if (f->k % 16 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0) {
-    // Rows TMA cannot address: copied once into rows of k_pad bytes (the filter is zero there, so what the tail of a
-    // row holds does not matter).  One thread per output over the rows as they are took 670 us on 3200 x 1592 x 320.
-    const size_t need = static_cast<size_t>(m) * f->k_pad;
-    lda = f->k_pad;
-    tc = may_stage(ctx, need);  // (else: the CUDA-core kernel below)
-    if (tc) {
-      int rc = ctx->reserve(align_up(need, 256));
+  const bool copy = f->k % 16 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0;
+  const FcPath path = fc_path(f, x, m, mode, copy);
+  if (path == FC_FEW_ROWS) return fc_few_rows_launch(ctx, x, m, f->k, f->wt.as<int8_t>(), f->k_pad, f->n, mode, y, e);
+  if (path == FC_TENSOR) {
+    const int8_t* rows = x;
+    int lda = f->k;
+    if (copy) {
+      // Rows TMA cannot address: copied once into rows of k_pad bytes (the filter is zero there, so what the tail of a
+      // row holds does not matter).
+      int rc = ctx->reserve(align_up(static_cast<size_t>(m) * f->k_pad, 256));
       if (rc) return rc;
       if ((rc = pitch_rows_i8_launch(ctx, x, ctx->ws, m, f->k, f->k_pad))) return rc;
       rows = static_cast<const int8_t*>(ctx->ws);
+      lda = f->k_pad;
     }
-  }
-  if (tc) {
     IgemmProblem p;
     memset(&p, 0, sizeof(p));
     p.a = rows; p.im2col = 0; p.cin_pad = f->k_pad; p.lda = lda; p.kh = p.kw = 1;
@@ -1046,15 +1077,18 @@ static int fc_run_mode(plb_fc* f, const int8_t* x, void* y, int m, int mode) {
     p.sw = &f->sw;
     return igemm_tc_launch(ctx, p, f->plans);
   }
+  // The threads of a warp read the rows of neighbouring outputs: from rows of whole 32-byte groups that would be bank conflicts
+  // in L1 (25 x 1012 x 174: 38 us, 15 from rows of k bytes).
+  const bool padded = f->w_rows.p == nullptr;
   ConvGeom g;
   memset(&g, 0, sizeof(g));
   g.batch = m; g.cin = f->k; g.h = 1; g.w = 1; g.cin_stride = f->k; g.cout = f->n; g.kh = g.kw = 1;
-  g.stride_h = g.stride_w = 1; g.dil_h = g.dil_w = 1; g.groups = 1; g.ho = g.wo = 1; g.cg_pad = f->k_pad;
+  g.stride_h = g.stride_w = 1; g.dil_h = g.dil_w = 1; g.groups = 1; g.ho = g.wo = 1; g.cg_pad = padded ? f->k_pad : f->k;
   g.dw_strip = -1;
   OutSpec o;
   memset(&o, 0, sizeof(o));
   o.mode = mode; o.y = y; o.ldy = f->n; o.epi = e;
-  return conv_direct_launch(ctx, g, x, f->wt.as<int8_t>(), o);
+  return conv_direct_launch(ctx, g, x, padded ? f->wt.as<int8_t>() : f->w_rows.as<int8_t>(), o);
 }
 
 int plb_fc_run(plb_fc* fc, const int8_t* x, void* y, int m) {

@@ -172,10 +172,34 @@ def test_fc_row_lengths(plb, ctx, m, k, n):
         assert np.array_equal(q.cpu().numpy(), q_ref)
 
 
+# both sides of each line of the choice between the filter pass, one thread per output and tiles (behind a copy of the rows,
+# which is a launch of its own)
+@pytest.mark.parametrize("m,k,n,offset,launches", [
+    (8, 512, 1000, 0, 1), (8, 2048, 1000, 0, 1), (4, 2048, 1000, 0, 1), (4, 8192, 64, 0, 1),   # filter pass, tiles
+    (8, 4100, 64, 0, 2), (2, 4100, 64, 0, 1), (8, 8192, 64, 4, 2),                             # ... with a copy
+    (185, 108, 110, 0, 1), (600, 428, 330, 0, 2), (103, 316, 518, 0, 2), (514, 116, 58, 4, 1),  # one thread, copy and tiles
+    (100, 1232, 512, 0, 1), (100, 112, 33, 0, 1),                                              # rows TMA addresses, k % 32 == 16
+])
+def test_fc_path_choice(plb, ctx, m, k, n, offset, launches):
+    x, wq, ws, bias = fc_case(m + k + n, m, k, n)
+    acc_ref = O.fc_acc_i32(x, wq)
+    fc = plb.Fc(ctx, wq, ws, 0.02, bias, O.ACT_RELU, out_scale=0.05)
+    xd = torch.empty(m * k + offset, dtype=torch.int8, device="cuda")[offset:].view(m, k)
+    xd.copy_(dev(x))
+    before = ctx.launch_count()
+    q = fc.run(xd)
+    ctx.sync()
+    assert ctx.launch_count() - before == launches
+    assert np.array_equal(q.cpu().numpy(), O.epilogue(acc_ref, ws, 0.02, bias, O.ACT_RELU, 0.0, out_scale=0.05))
+    y = plb.Fc(ctx, wq, ws, 0.02, bias, O.ACT_RELU).run(xd)
+    ctx.sync()
+    assert np.array_equal(y.cpu().numpy(), O.epilogue(acc_ref, ws, 0.02, bias, O.ACT_RELU, 0.0))
+
+
 def test_fc_captured_call_keeps_no_scratch(plb):
     """A graph of a layer whose rows are copied in an ordinary call (k % 16 != 0) stays good when the ctx workspace is
     replaced by a larger one afterwards: the captured call does not use it."""
-    m, k, n = 40, 100, 64
+    m, k, n = 400, 1000, 64
     x, wq, ws, bias = fc_case(5, m, k, n)
     want = O.epilogue(O.fc_acc_i32(x, wq), ws, 0.02, bias, O.ACT_NONE, 0.0)
     stream = torch.cuda.Stream()
@@ -187,6 +211,7 @@ def test_fc_captured_call_keeps_no_scratch(plb):
         fc.run(xd, out=y)
         own.sync()
         size = own.workspace_size()
+        assert size >= m * k
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g, stream=stream):
             fc.run(xd, out=y)
@@ -201,7 +226,7 @@ def test_fc_captured_call_keeps_no_scratch(plb):
 
 def test_fc_small_caller_workspace(plb):
     """A workspace of the caller's that is too small for the copy of the rows: the layer runs without it."""
-    m, k, n = 40, 100, 64
+    m, k, n = 400, 1000, 64
     x, wq, ws, bias = fc_case(6, m, k, n)
     own = plb.Context(0)
     own.set_workspace(torch.empty(1024, dtype=torch.uint8, device="cuda"))
