@@ -1477,6 +1477,7 @@ TcSwitches tc_switches_from_env() {
   s.dwpw = env_int("PLB_DWPW", -1);
   s.dwpw_tw = env_int("PLB_DWPW_TW", -1);
   s.dwpw_seg = env_int("PLB_DWPW_SEG", -1);
+  s.sparse_tmem = env_int("PLB_SPARSE_TMEM", -1);
   return s;
 }
 

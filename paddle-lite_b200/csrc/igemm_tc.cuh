@@ -36,6 +36,7 @@ struct TcSwitches {
   int dwpw = -1;          // PLB_DWPW=0: depthwise + 1x1 pairs never run as one launch
   int dwpw_tw = -1;       // PLB_DWPW_TW: tile columns of the fused depthwise + 1x1 kernel (4 / 8 / 16)
   int dwpw_seg = -1;      // PLB_DWPW_SEG: output rows per work item of that kernel
+  int sparse_tmem = -1;   // PLB_SPARSE_TMEM: fp32 sparse layers never (0) / always (1) with their activations in tensor memory
 };
 TcSwitches tc_switches_from_env();
 

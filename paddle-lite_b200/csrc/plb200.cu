@@ -240,7 +240,7 @@ struct plb_sparse {
   DeviceBuf row_ptr, col, val, bias_raw;
   DeviceBuf col_val;  // fp32: {input channel, weight bits} per non-zero
   DeviceBuf tmem_rows, tmem_batches;  // fp32: the non-zeros as sparse_tmem.cu walks them (empty: it cannot take this layer)
-  int tmem_pixels = 0;
+  int tmem_pixels = 0, tmem_switch = -1;
   DeviceBuf grp_ptr, grp_idx, grp_w;  // int8: non-zeros in groups of four for the slab kernel
   DeviceBuf scale, bias;
   float alpha = 0.f;
@@ -332,6 +332,7 @@ long plb_ctx_launch_count(const plb_ctx* ctx) { return ctx ? ctx->launches : 0; 
 long plb_ctx_window_launch_count(const plb_ctx* ctx) { return ctx ? ctx->window_launches : 0; }
 long plb_ctx_nchw_launch_count(const plb_ctx* ctx) { return ctx ? ctx->nchw_launches : 0; }
 long plb_ctx_nchw_gather_launch_count(const plb_ctx* ctx) { return ctx ? ctx->nchw_gather_launches : 0; }
+long plb_ctx_sparse_tmem_launch_count(const plb_ctx* ctx) { return ctx ? ctx->sparse_tmem_launches : 0; }
 long plb_ctx_stem_launch_count(const plb_ctx* ctx) { return ctx ? ctx->stem_launches : 0; }
 long plb_ctx_dwpw_launch_count(const plb_ctx* ctx) { return ctx ? ctx->dwpw_launches : 0; }
 long plb_ctx_pair_launch_count(const plb_ctx* ctx) { return ctx ? ctx->pair_launches : 0; }
@@ -1215,6 +1216,7 @@ int plb_sparse_prepare(plb_ctx* ctx, const plb_sparse_desc* desc, const void* no
     SparseTmemLists lists;
     if (sparse_tmem_build(d.cin, d.cout, static_cast<long>(d.h) * d.w, row_ptr, col, valf, bias_h, &lists)) {
       s->tmem_pixels = lists.pixels;
+      s->tmem_switch = tc_switches_from_env().sparse_tmem;
       if ((rc = s->tmem_rows.upload(lists.rows.data(), lists.rows.size() * sizeof(int4)))) return rc;
       if ((rc = s->tmem_batches.upload(lists.batches.data(), lists.batches.size() * sizeof(int)))) return rc;
     }
@@ -1295,7 +1297,7 @@ int plb_sparse_run(plb_sparse* sp, const void* x, void* y, int batch) {
     p.batch = batch; p.cin = g.cin; p.cout = g.cout; p.hw = g.hw; p.pixels = sp->tmem_pixels; p.nnz = sp->nnz;
     p.x = static_cast<const float*>(x); p.rows = sp->tmem_rows.p; p.batches = sp->tmem_batches.p;
     p.act = e.act; p.alpha = e.alpha; p.y = static_cast<float*>(y);
-    if (sparse_tmem_better(p)) return sparse_tmem_launch(sp->ctx, p);
+    if (sp->tmem_switch < 0 ? sparse_tmem_better(p, sp->ctx->sm_count) : sp->tmem_switch != 0) return sparse_tmem_launch(sp->ctx, p);
   }
   return sparse_csr_launch(sp->ctx, g, x, sp->row_ptr.as<int>(), sp->col.as<int>(), sp->val.p, sp->col_val.p,
                            sp->bias_raw.as<float>(), e, y);

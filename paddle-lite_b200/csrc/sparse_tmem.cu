@@ -2,7 +2,8 @@
 //
 // Per non-zero and pixel the walk reads one activation and does one multiply-add.  Out of shared memory that read is the
 // bound: 4 bytes per multiply-add against 128 bytes per clock and SM keep the FMA pipes a quarter busy.  Tensor memory
-// delivers more than that to EACH of the four schedulers, so the activations live there: lane = pixel, column =
+// delivers 43 to 85 bytes per clock to each of the four schedulers (loads of four and eight columns, as measured below),
+// 170 to 340 to the SM, so the activations live there: lane = pixel, column =
 // (input channel, pixel group).  One tcgen05.ld of four (eight) columns gives every lane of a warp four (eight) pixels of one
 // channel -- the column address is the non-zero's channel -- and feeds as many multiply-adds per lane.
 //
@@ -387,19 +388,64 @@ bool sparse_tmem_build(int cin, int cout, long hw, const std::vector<int>& row_p
   return true;
 }
 
-bool sparse_tmem_better(const SparseTmemProblem& p) {
-  const bool vec = p.hw % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.y)) & 15) == 0;
-  if (vec && p.cin <= 512) {
-    // against the shared-memory tiles: just above 128 channels a second chunk moves every partial sum twice for few
-    // non-zeros (137 -> 288 on 98 x 98, 47 images: 885 us against 838; 256 -> 256 on 28 x 28, 256 images: 497 against 799)
-    return p.cin <= 128 || p.cin > 160;
+namespace {
+
+bool aligned16(const SparseTmemProblem& p) {
+  return p.hw % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.y)) & 15) == 0;
+}
+
+// Few pixel groups: several teams share one, each with a slice of the output channels (and its own copy of the activations).
+// The number of slices that finishes first by the cycles of a load, a non-zero and a row.
+struct Split {
+  int slices;
+  long waves;  // items per team, rounded up
+};
+Split split(const SparseTmemProblem& p, int sm_count) {
+  const int chunks = (p.cin + 512 / p.pixels - 1) / (512 / p.pixels);
+  const long groups = (static_cast<long>(p.batch) * p.hw + 32 * p.pixels - 1) / (32 * p.pixels), teams = 4L * sm_count;
+  Split best = {1, 1};
+  double best_cost = 0;
+  for (int s = 1; s <= 64 && (s == 1 || s * kTeamWarps <= p.cout); ++s) {
+    const long waves = (groups * s + teams - 1) / teams;
+    const double cost = waves * (5.0 * p.pixels * p.cin + 3.0 * p.pixels * p.nnz / s + 60.0 * chunks * ((p.cout + s - 1) / s));
+    if (s == 1 || cost < best_cost) {
+      best_cost = cost;
+      best = {s, waves};
+    }
   }
-  if (p.cin <= 160) return true;  // against whole channels of a few pixels per thread: 130 -> 70 on 19 x 23, 64 images: 41 us against 135
-  // Against one thread per output: its launch takes as long as one thread's walk (0.13 us per non-zero), or 0.64 us per
-  // million non-zeros and pixels; a chunk takes at least 8 us here (1024 -> 1024 on 7 x 7: 119 us against 29 for one image,
-  // 596 against 1694 for 256; 1000 -> 500 on 13 x 11, 20 images: 127 against 174).
-  const double plain = 3 + std::max(0.13 * p.nnz / p.cout, 0.64e-6 * p.nnz * p.batch * p.hw);
-  return 8.0 * ((p.cin + 512 / p.pixels - 1) / (512 / p.pixels)) < plain;
+  return best;
+}
+
+}  // namespace
+
+// Costs in us, fitted to 500 layers (32 to 1024 channels, 4 to 112 pixels a side, 1 to 256 images, densities 0.05 to 0.35); the
+// choice is 0.2 % from the faster kernel over all of them.  Measured, here / the other one: 137 -> 288 on 98 x 98, 47 images
+// 885 / 838; 160 -> 220 on 16 x 16, 164 images 59 / 47, but 159 -> 160 on 9520 pixels, 2 images 26 / 34; 329 -> 43 on 16 x 16,
+// 7 images 12.9 / 8.8; 192 -> 82 on 5 x 5, 12 images 16 / 4.9; 448 -> 150 on 4225 pixels, 4 images 100 / 196.
+bool sparse_tmem_better(const SparseTmemProblem& p, int sm_count) {
+  const bool vec = aligned16(p), tiles = vec && p.cin <= 512;
+  if (p.batch > 65535 || (!tiles && p.cout > 65535)) return true;  // beyond the other kernels' grids
+  // against whole channels of a few pixels per thread: 130 -> 70 on 19 x 23, 64 images 41 / 135; faster on all 115 measured
+  if (!tiles && p.cin <= 160) return true;
+  const int chunks = (p.cin + 512 / p.pixels - 1) / (512 / p.pixels);
+  const Split sp = split(p, sm_count);
+  const double w = static_cast<double>(sp.waves), nnz = static_cast<double>(p.nnz);
+  const double load = w * p.pixels * p.cin, walk = w * p.pixels * nnz / sp.slices;
+  const double rows = w * chunks * ((p.cout + sp.slices * kTeamWarps - 1) / (sp.slices * kTeamWarps));
+  const double partial = (chunks - 1.0) * p.batch * p.hw * p.cout;  // sums that wait in y
+  const double here = vec ? 3.0 + 4.8e-3 * load + 2.0e-3 * walk + 0.36 * rows + 0.54 * chunks + 5.8e-7 * partial
+                          : 3.8 + 1.01e-2 * load + 1.9e-3 * walk + 0.52 * rows + 0.79 * chunks + 3.3e-7 * partial + 0.38 * w;
+  double there;
+  if (tiles) {  // tiles of 4 * pg pixels in shared memory, two blocks per SM: every block walks all non-zeros
+    const int pg = p.cin <= 128 ? 32 : p.cin <= 256 ? 16 : 8;
+    const long blocks = static_cast<long>(p.batch) * ((p.hw + 4 * pg - 1) / (4 * pg)), slots = 2L * sm_count;
+    const double walks = static_cast<double>((blocks + slots - 1) / slots) * nnz;
+    there = 0.95 * (pg == 32 ? 5.1 + 1.06e-2 * walks : pg == 16 ? 5.6 + 5.5e-3 * walks : 8.5 + 3.0e-3 * walks);
+  } else {  // one thread per output
+    there = 2.6 + 0.067 * nnz / p.cout + 4.75e-7 * nnz * p.batch * ((p.hw + 31) / 32 * 32) +
+            4.7e-4 * p.cout * p.batch * ((p.hw + 255) / 256);
+  }
+  return here < there;
 }
 
 int sparse_tmem_launch(plb_ctx* ctx, const SparseTmemProblem& p) {
@@ -410,26 +456,17 @@ int sparse_tmem_launch(plb_ctx* ctx, const SparseTmemProblem& p) {
   const int channels = 512 / p.pixels;
   a.chunks = (p.cin + channels - 1) / channels;
   if (a.pixels == 0) return PLB_OK;
-  // Few pixel groups: several teams share one, each with a slice of the output channels (and its own copy of the
-  // activations).  The number of slices that finishes first by the cycles of a load, a non-zero and a row.
   const long groups = (a.pixels + 32 * p.pixels - 1) / (32 * p.pixels), teams = 4L * ctx->sm_count;
-  double best = 0;
-  for (int s = 1; s <= 64 && (s == 1 || s * kTeamWarps <= p.cout); ++s) {
-    const double waves = static_cast<double>((groups * s + teams - 1) / teams);
-    const double cost = waves * (5.0 * p.pixels * p.cin + 3.0 * p.pixels * p.nnz / s + 60.0 * a.chunks * ((p.cout + s - 1) / s));
-    if (s == 1 || cost < best) {
-      best = cost;
-      a.slices = s;
-    }
-  }
+  a.slices = split(p, ctx->sm_count).slices;
   if (groups * a.slices + teams > 0x7fffffffL) return fail(PLB_E_UNSUPPORTED, "sparse grid too large");
   a.items = static_cast<int>(groups * a.slices);
-  const bool vec = p.hw % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.y)) & 15) == 0;
+  const bool vec = aligned16(p);
   Kernel kern = p.pixels == 8 ? (vec ? pick<8, true>(p.act) : pick<8, false>(p.act))
                               : (vec ? pick<4, true>(p.act) : pick<4, false>(p.act));
   PLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes));
   PLB_CUDA(launch_kernel(kern, dim3(std::min<long>(a.items, ctx->sm_count)), dim3(kThreads), kStageBytes, ctx->stream, a));
   ctx->launches++;
+  ctx->sparse_tmem_launches++;
   return PLB_OK;
 }
 

@@ -33,7 +33,7 @@ struct SparseTmemProblem {
   float* y;           // [batch, cout, hw]
 };
 // Whether it is the faster kernel for these sizes and addresses.
-bool sparse_tmem_better(const SparseTmemProblem& p);
+bool sparse_tmem_better(const SparseTmemProblem& p, int sm_count);
 int sparse_tmem_launch(plb_ctx* ctx, const SparseTmemProblem& p);
 
 }  // namespace plb

@@ -105,10 +105,10 @@ def test_sparse_fp32_row_lengths(plb, ctx, cin, cout, h, w, batch, act, alpha):
         assert np.array_equal(yd.cpu().numpy(), y_ref)
 
 
-def test_sparse_fp32_special_values(plb, ctx):
+def special_values(plb, ctx, cin, hw):
     """Only the non-zeros take part: infinities and NaN in a channel reach exactly the outputs that read it, and a sum of
     negative zeros stays one."""
-    cin, cout, hw = 150, 12, 6
+    cout = 12
     rng = np.random.default_rng(3)
     wf = np.where(rng.random((cout, cin)) < 0.1, rng.standard_normal((cout, cin)), 0).astype(np.float32)
     wf[3, :] = 0
@@ -125,6 +125,50 @@ def test_sparse_fp32_special_values(plb, ctx):
     ok = ~np.isnan(y_ref)
     assert np.array_equal(y[ok].view(np.int32), y_ref[ok].view(np.int32))
     assert np.all(np.signbit(y[:, 3]))
+
+
+def test_sparse_fp32_special_values(plb, ctx):
+    special_values(plb, ctx, 150, 6)
+
+
+# The two tests above on the tensor-memory kernel whatever the choice between kernels says: 1, 2, 3 and 5 chunks of channels,
+# on and off the 16-byte grid.
+@pytest.mark.parametrize("cin,cout,h,w,batch", [(60, 23, 4, 4, 40), (129, 30, 8, 4, 9), (300, 41, 3, 11, 5), (300, 41, 4, 12, 5),
+                                                (640, 9, 7, 7, 12), (640, 26, 8, 8, 3)])
+@pytest.mark.parametrize("act,alpha", [(0, 0.0), (2, 1.5), (3, 0.1)])
+def test_sparse_fp32_row_lengths_in_tensor_memory(plb, ctx, monkeypatch, cin, cout, h, w, batch, act, alpha):
+    monkeypatch.setenv("PLB_SPARSE_TMEM", "1")
+    before = ctx.sparse_tmem_launch_count()
+    test_sparse_fp32_row_lengths(plb, ctx, cin, cout, h, w, batch, act, alpha)
+    assert ctx.sparse_tmem_launch_count() == before + 2
+
+
+@pytest.mark.parametrize("cin,hw", [(150, 6), (150, 5), (300, 6), (600, 6), (600, 5)])
+def test_sparse_fp32_special_values_in_tensor_memory(plb, ctx, monkeypatch, cin, hw):
+    monkeypatch.setenv("PLB_SPARSE_TMEM", "1")
+    before = ctx.sparse_tmem_launch_count()
+    special_values(plb, ctx, cin, hw)
+    assert ctx.sparse_tmem_launch_count() == before + 1
+
+
+# (cin, cout, h, w, batch, density, kernel): both sides of the lines between tensor memory, shared-memory tiles and one thread
+# per output
+@pytest.mark.parametrize("cin,cout,h,w,batch,density,tmem", [
+    (489, 33, 18, 18, 2, 0.08, False), (128, 46, 30, 30, 17, 0.1, True), (329, 43, 16, 16, 7, 0.06, False),
+    (192, 82, 5, 5, 12, 0.15, False), (224, 101, 5, 5, 2, 0.31, False), (448, 150, 33, 33, 4, 0.3, True), (100, 40, 5, 5, 3, 0.2, True),
+])
+def test_sparse_fp32_kernel_choice(plb, ctx, cin, cout, h, w, batch, density, tmem):
+    rng = np.random.default_rng(cin)
+    wf = np.where(rng.random((cout, cin)) < density, rng.standard_normal((cout, cin)), 0).astype(np.float32)
+    x = rng.standard_normal((batch, cin, h, w)).astype(np.float32)
+    bias = rng.standard_normal(cout).astype(np.float32)
+    enc = O.sparse_encode(wf, h * w)
+    before = ctx.sparse_tmem_launch_count()
+    y = plb.SparseConv(ctx, enc["nonzero_weights"], enc["oc_nonzeros"], enc["diffs"], enc["first_ic"], enc["flag_semi"],
+                       cin=cin, cout=cout, in_hw=(h, w), bias=bias, act=O.ACT_RELU).run(dev(x))
+    ctx.sync()
+    assert ctx.sparse_tmem_launch_count() - before == (1 if tmem else 0)
+    assert np.array_equal(y.cpu().numpy(), O.sparse_conv_f32(x, wf, bias, O.ACT_RELU))
 
 
 # the sparse_conv benchmark shapes: MobileNetV1 pointwise layers at batch 256, 80 % of the weights masked
