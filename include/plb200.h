@@ -68,7 +68,7 @@ int plb_ctx_sync(plb_ctx* ctx);
  * a device share (at most 512 MB of it unused, none when the last context is gone).  Replaces the
  * per-Run TargetMalloc of the im2col buffer (conv_compute.cc:306-310). */
 int plb_ctx_set_workspace(plb_ctx* ctx, void* dptr, size_t bytes);
-/* Bytes of scratch the NCHW entry points of this object need for `batch` images. */
+/* Bytes of scratch that are enough for every NCHW entry point of this object and `batch` images (a call may use less). */
 size_t plb_conv_workspace_bytes(const plb_conv* conv, int batch);
 const char* plb_last_error(void);
 /* Number of kernels this library has launched on the ctx since creation. */

@@ -500,15 +500,23 @@ static size_t staged_input_bytes(const plb_conv* conv, int batch) {
   return align_up(static_cast<size_t>(batch) * pixels * conv->cin_pad, 256);
 }
 
+// bytes of the rows of a padded pitch that 1x1 layers on images whose pixel count is not a multiple of 16 may stage instead
+static size_t pitched_bytes(const plb_conv* conv, int batch) {
+  const size_t hwp = align_up(static_cast<size_t>(conv->d.h) * conv->d.w, 16);
+  return align_up(static_cast<size_t>(batch) * conv->d.cin * hwp, 256) +
+         align_up(static_cast<size_t>(batch) * conv->d.cout * hwp * 4, 256);
+}
+
+// What a call that stages uses: tensor-core layers write their results themselves (but for the two-SM tiles, only when forced).
+static bool stages_output(const plb_conv* conv) { return conv->kind != 0 || conv->sw.pair == 1; }
+static size_t staged_bytes(const plb_conv* conv, int batch, bool output) {
+  const size_t y_bytes = align_up(static_cast<size_t>(batch) * conv->ho * conv->wo * conv->d.cout * 4, 256);
+  return staged_input_bytes(conv, batch) + (output ? y_bytes : 0);
+}
+
 size_t plb_conv_workspace_bytes(const plb_conv* conv, int batch) {
   if (!conv || batch <= 0) return 0;
-  const size_t x_bytes = staged_input_bytes(conv, batch);
-  const size_t y_bytes = align_up(static_cast<size_t>(batch) * conv->ho * conv->wo * conv->d.cout * 4, 256);
-  // 1x1 layers on images whose pixel count is not a multiple of 16 stage rows of a padded pitch instead
-  const size_t hwp = align_up(static_cast<size_t>(conv->d.h) * conv->d.w, 16);
-  const size_t pitched = align_up(static_cast<size_t>(batch) * conv->d.cin * hwp, 256) +
-                         align_up(static_cast<size_t>(batch) * conv->d.cout * hwp * 4, 256);
-  return std::max(x_bytes + y_bytes, pitched);
+  return std::max(staged_bytes(conv, batch, true), pitched_bytes(conv, batch));
 }
 
 int plb_softmax_f32(plb_ctx* ctx, const float* x, float* y, int rows, int cols) {
@@ -676,10 +684,11 @@ NchwPath nchw_path(const plb_conv* c, const int8_t* x, void* y, int batch, int m
   NchwPath path;
   if (c->sw.nchw == 1)
     path = can_gather ? NCHW_GATHERED : NCHW_PITCHED;
-  else if (can_gather && !may_stage(c->ctx, plb_conv_workspace_bytes(c, batch)))
-    path = NCHW_GATHERED;  // (the one that needs no scratch)
   else
     path = path_1x1_odd(c->ctx, *p, can_gather, g);
+  if (path != NCHW_GATHERED && can_gather && c->sw.nchw != 1 &&
+      !may_stage(c->ctx, path == NCHW_PITCHED ? pitched_bytes(c, batch) : staged_bytes(c, batch, stages_output(c))))
+    path = NCHW_GATHERED;  // (the one that needs no scratch)
   if (path == NCHW_PITCHED) {
     // the caller stages x and y with rows a multiple of 16 bytes apart and fills in the addresses
     if (p->cin_pad % 32 != 0 || (reinterpret_cast<uintptr_t>(y) & 15) != 0) return NCHW_STAGED;
@@ -704,7 +713,7 @@ int conv_run_nchw(plb_conv* c, const int8_t* x, void* y, int batch, int mode) {
       // pixel counts that are not a multiple of 16: re-pitch the rows into the workspace, run, copy back
       const int eb = mode == OUT_I8 ? 1 : 4;
       const size_t xs_bytes = align_up(static_cast<size_t>(batch) * d.cin * np.x_pitch, 256);
-      int rc = ctx->reserve(plb_conv_workspace_bytes(c, batch));
+      int rc = ctx->reserve(pitched_bytes(c, batch));
       if (rc) return rc;
       uint8_t* base = static_cast<uint8_t*>(ctx->ws);
       np.x = reinterpret_cast<const int8_t*>(base);
@@ -719,7 +728,7 @@ int conv_run_nchw(plb_conv* c, const int8_t* x, void* y, int batch, int mode) {
     if (dw_nchw_supported(g, mode)) return dw_nchw_launch(ctx, g, x, c->w.as<int8_t>(), out_spec(c, mode, y));
   }
   const size_t x_bytes = staged_input_bytes(c, batch);
-  int rc = ctx->reserve(plb_conv_workspace_bytes(c, batch));
+  int rc = ctx->reserve(staged_bytes(c, batch, stages_output(c)));
   if (rc) return rc;
   int8_t* xs = static_cast<int8_t*>(ctx->ws);
   void* ys = static_cast<uint8_t*>(ctx->ws) + x_bytes;
@@ -729,9 +738,8 @@ int conv_run_nchw(plb_conv* c, const int8_t* x, void* y, int batch, int mode) {
   else
     rc = nchw_to_nhwc_i8_launch(ctx, x, xs, batch, d.cin, d.h, d.w, c->cin_pad);
   if (rc) return rc;
-  // The tensor-core kernel writes NCHW itself; the two-SM tiles (only when forced here) and the CUDA-core kernels write
-  // channels-last into the workspace.
-  if (c->kind == 0 && c->sw.pair != 1) {
+  // The tensor-core kernel writes NCHW itself; the two-SM tiles and the CUDA-core kernels write channels-last into the workspace.
+  if (!stages_output(c)) {
     OutSpec o = out_spec(c, mode, y);
     o.y_nchw = 1;
     return conv_core(c, xs, batch, o);

@@ -291,6 +291,23 @@ def test_nchw_more_images_than_a_grid_dimension(plb, ctx, cin, cout, k, act):
     assert bool(same.all())
 
 
+def test_staged_layers_reserve_what_they_use(plb):
+    """A tensor-core layer stages its input only: a caller's workspace of that size is enough, and the context's own grows to
+    no more."""
+    xq, in_s, wq, ws, bias = conv_case(71, 3, 40, 17, 15, 48, 3)
+    want = O.conv_int8(xq, wq, ws, in_s, bias, O.ACT_RELU, pads=(1, 1, 1, 1))
+    need = (3 * 17 * 15 * 64 + 255) // 256 * 256
+    for own in (False, True):
+        c = plb.Context(0)
+        if not own:
+            c.set_workspace(torch.empty(need, dtype=torch.uint8, device="cuda"))
+        conv = plb.Conv(c, wq, ws, in_s, bias, in_hw=(17, 15), pads=(1, 1, 1, 1), act=plb.ACT_RELU)
+        y = conv.run(dev(xq))
+        c.sync()
+        assert np.array_equal(y.cpu().numpy(), want)
+        assert c.workspace_size() == need <= conv.workspace_bytes(3)
+
+
 def test_nchw_1x1_without_scratch(plb):
     """1x1 layers on planes TMA cannot address need no workspace: a caller's that is too small, and captured calls."""
     xq, in_s, wq, ws, bias = conv_case(12, 4, 64, 14, 14, 96, 1)
